@@ -1,0 +1,339 @@
+// dmf_async.cuh -- barrier-free relabel and push phases for deep graphs, part
+// of the solve kernel (included by dmf_kernel.cuh inside namespace dmfk).
+//
+// A grid-like graph of diameter D costs the level-synchronous phases about D
+// grid barriers per global relabel and as many per run of push rounds, each
+// with a few hundred vertices of work: 8.1 us a BFS level and 13 us a push
+// round on the 256 x 256 grid, nearly all of it barrier and dependent loads.
+// Here every vertex belongs to one lane for the whole phase (a warp owns
+// windows of 32 consecutive vertices), the lane polls the vertex's word in L2
+// and acts when it changes, and the grid meets at a barrier only when the phase
+// ends.  A hop then costs one poll and one fire-and-forget atomic: 0.8 us a BFS
+// level.  256 x 256 grid, one B200: static solve 145 -> 22 ms, 1% batch
+// 126 -> 15 ms.
+#pragma once
+
+// BFS levels after which a global relabel (and then the rest of the solve)
+// goes over to the barrier-free phases.  R-MAT graphs end within 10 levels:
+// there a level is real work and the worklists save polling every vertex.  A
+// graph that needs 24 levels will need hundreds of short phases.
+constexpr int kDeepLevels = 24;
+// Windows of 32 vertices per warp at most: bounds the vertices a graph may
+// have (kAsyncWin * 32 * resident warps) and the per-vertex shared memory.
+constexpr int kAsyncWin = 4;
+// Polls without work after which a warp counts as idle: longer than an atomic
+// takes to become visible, so that a wave crossing from one block to another
+// does not find every block idle.
+constexpr int kQuietPolls = 8;
+// Polls per phase at most (bounds the loop; a phase is far shorter).
+constexpr int kMaxPolls = 1 << 20;
+
+struct AsyncShared {
+  int scan[kAsyncWin * kBlock];  // label the vertex's arcs were last relaxed from
+  int idle_warps;
+  int stop;
+};
+
+__device__ __forceinline__ int ld_rlx(const int *p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ long long ld_rlx(const long long *p) {
+  long long v;
+  asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// The windows of a warp: block b owns `per` consecutive windows, warp i of it
+// windows i, i + warps, ...
+struct AsyncOwn {
+  int first, count;  // this warp's first vertex and its windows
+  int step;          // vertices from one window of the warp to the next
+};
+
+__device__ __forceinline__ AsyncOwn async_own(int n) {
+  const int nw = blockDim.x >> 5, wid = threadIdx.x >> 5;
+  const int nwin = (n + 31) >> 5, per = (nwin + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int lo = blockIdx.x * per + wid, hi = min(nwin, (int)(blockIdx.x + 1) * per);
+  AsyncOwn o;
+  o.first = lo * 32;
+  o.step = nw * 32;
+  o.count = lo < hi ? (hi - lo + nw - 1) / nw : 0;
+  return o;
+}
+
+// Whether the grid's warps can own every vertex.
+__device__ __forceinline__ bool async_fits(int n) {
+  const int nwin = (n + 31) >> 5, per = (nwin + (int)gridDim.x - 1) / (int)gridDim.x;
+  return per <= kAsyncWin * (int)(blockDim.x >> 5);
+}
+
+// Quiescence: a warp is idle after kQuietPolls polls without work, a block when
+// all its warps are, and the phase ends once every block is idle (or *stop is
+// set).  This may end a phase too early (work in flight to an idle block); the
+// relabel checks its labels after a barrier, and a push phase may end at any
+// time.  One poll of the grid-wide words per block and 8 polls.
+struct AsyncIdle {
+  int quiet = 0;
+  bool idle = false;
+};
+
+__device__ __forceinline__ void async_begin(AsyncShared &sh) {
+  if (threadIdx.x == 0) {
+    sh.idle_warps = 0;
+    sh.stop = 0;
+  }
+  __syncthreads();
+}
+
+// A warp that found work in its last poll.
+__device__ __forceinline__ bool async_busy(AsyncShared &sh, AsyncIdle &st, int *idle_blocks) {
+  st.quiet = 0;
+  if (st.idle) {
+    st.idle = false;
+    if ((threadIdx.x & 31) == 0 && atomicSub(&sh.idle_warps, 1) == (int)(blockDim.x >> 5)) atomicSub(idle_blocks, 1);
+  }
+  return *(volatile int *)&sh.stop != 0;
+}
+
+// A warp whose last poll found nothing; true: leave the phase.  The block's
+// first warp looks at the grid-wide words.  The SM's warps share its issue
+// slots, so a poll is kept short and a warp without vertices sleeps.
+__device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool owner, int poll, int *idle_blocks,
+                                            const int *stop, const int *err) {
+  if (++st.quiet < kQuietPolls && owner) return false;
+  if (!st.idle) {
+    st.idle = true;
+    if ((threadIdx.x & 31) == 0 && atomicAdd(&sh.idle_warps, 1) == (int)(blockDim.x >> 5) - 1)
+      atomicAdd(idle_blocks, 1);
+  }
+  if (threadIdx.x == 0 && (st.quiet & 3) == 0 &&
+      (ld_rlx(idle_blocks) >= (int)gridDim.x || ld_rlx(stop) || ld_rlx(err) || poll >= kMaxPolls))
+    *(volatile int *)&sh.stop = 1;
+  if (!owner) __nanosleep(200);
+  return *(volatile int *)&sh.stop != 0;
+}
+
+// Global relabel from the labels a level-synchronous BFS left after its level
+// L0 (seeds only: L0 = 0): label-correcting, every vertex relaxes the tails of
+// its residual in-arcs with an atomic minimum whenever its own label fell.
+// Labels only fall and every fall is seen by its owner, so once no vertex has a
+// label below the one it last relaxed from (ph_async_settled, between two
+// barriers) the labels are the exact distances.
+template <int W>
+__device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh, const AsyncOwn &own, int L0, bool first,
+                                               LStats &ls) {
+  Ctrl *c = p.ctrl;
+  const int lane = threadIdx.x & 31;
+  int scan[W], beg[W];
+  unsigned mask[W];  // arcs (of degree <= 8) whose head can be labelled over them, and the degree << 8
+#pragma unroll
+  for (int j = 0; j < W; j++) {
+    const int v = own.first + j * own.step + lane;
+    scan[j] = INT_MIN;
+    beg[j] = 0;
+    mask[j] = 0;
+    if (j < own.count && v < p.n) {
+      const int h = __ldcg(p.height + v);
+      scan[j] = first ? h : sh.scan[j * kBlock + (int)threadIdx.x];
+      if (h != p.n && inst_on(p, v)) {        // neither a source nor dead
+        if (first && h == L0) scan[j] = UNV;  // the frontier
+        beg[j] = __ldg(p.off + v);
+        const int deg = __ldg(p.off + v + 1) - beg[j];
+        mask[j] = (unsigned)min(deg, 255) << 8;
+        if (deg <= kSmallMax) {
+#pragma unroll
+          for (int k = 0; k < kSmallMax; k++)
+            if (k < deg && __ldcg(p.res + __ldg(p.par + beg[j] + k)) > 0 &&
+                __ldcg(p.height + __ldg(p.adj + beg[j] + k)) != p.n)
+              mask[j] |= 1u << k;
+        }
+      }
+    }
+  }
+  AsyncIdle st;
+  for (int poll = 0;; poll++) {
+    int h[W];
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+      const int v = own.first + j * own.step + lane;
+      h[j] = j < own.count && v < p.n ? ld_rlx(p.height + v) : INT_MAX;
+    }
+    bool need_any = false;
+#pragma unroll
+    for (int j = 0; j < W; j++) need_any |= h[j] < scan[j];
+    if (!__any_sync(0xffffffffu, need_any)) {
+      if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[0], &c->astop, &c->err)) break;
+      continue;
+    }
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+      const bool need = h[j] < scan[j];
+      const unsigned deg = mask[j] >> 8;
+      if (need) {
+        scan[j] = h[j];
+        if (deg <= kSmallMax) {
+#pragma unroll
+          for (int k = 0; k < kSmallMax; k++)
+            if ((mask[j] >> k) & 1) atomicMin(p.height + __ldg(p.adj + beg[j] + k), h[j] + 1);
+          ls.barcs += deg;
+        }
+      }
+      unsigned wide = __ballot_sync(0xffffffffu, need && deg > kSmallMax);
+      while (wide) {  // longer rows by the whole warp
+        const int src = __ffs(wide) - 1;
+        wide &= wide - 1;
+        const int v = own.first + j * own.step + src;
+        const int b = __shfl_sync(0xffffffffu, beg[j], src), e = __ldg(p.off + v + 1);
+        const int hv = __shfl_sync(0xffffffffu, h[j], src);
+        for (int a = b + lane; a < e; a += 32) {
+          const int w = __ldg(p.adj + a);
+          ls.barcs++;
+          const int cur = __ldcg(p.height + w);
+          if (cur > hv + 1 && cur != p.n && __ldcg(p.res + __ldg(p.par + a)) > 0) atomicMin(p.height + w, hv + 1);
+        }
+        __syncwarp();
+      }
+    }
+    if (async_busy(sh, st, &c->aidle[0])) break;
+  }
+#pragma unroll
+  for (int j = 0; j < W; j++) sh.scan[j * kBlock + (int)threadIdx.x] = scan[j];
+}
+
+__device__ __forceinline__ void ph_async_bfs(const Params &p, AsyncShared &sh, int L0, bool first, LStats &ls) {
+  Ctrl *c = p.ctrl;
+  const AsyncOwn own = async_own(p.n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    c->aidle[1] = 0;  // the push phase's words
+    c->astop = 0;
+    c->aunsettled = 0;
+    c->aact = 0;
+    c->adepth = 0;
+  }
+  async_begin(sh);
+  if (own.count <= 1) async_bfs_loop<1>(p, sh, own, L0, first, ls);
+  else async_bfs_loop<kAsyncWin>(p, sh, own, L0, first, ls);
+}
+
+// After a barrier: counts the vertices whose label fell since they last relaxed
+// their arcs (0: the labels are exact).
+__device__ __forceinline__ void ph_async_settled(const Params &p, AsyncShared &sh) {
+  const AsyncOwn own = async_own(p.n);
+  const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.ctrl->aidle[0] = 0;
+  bool open = false;
+  for (int j = 0; j < own.count; j++) {
+    const int v = own.first + j * own.step + lane;
+    if (v < p.n) open |= __ldcg(p.height + v) < sh.scan[j * kBlock + (int)threadIdx.x];
+  }
+  if (__syncthreads_or(open) && threadIdx.x == 0) atomicAdd(&p.ctrl->aunsettled, 1);
+}
+
+// ph_bfs_finalize of a complete relabel, which also counts the active vertices
+// and finds the greatest distance.
+__device__ __forceinline__ void ph_async_finalize(const Params &p, bool write_side) {
+  int nd = 0, act = 0, depth = 0;
+  for_live_vertices<4>(p, [&](int v) {
+    const int h = __ldcg(p.height + v);
+    if (h == UNV) {
+      p.dead[v] = 1;
+      p.height[v] = p.n;
+      nd++;
+    } else if (h < p.n) {
+      depth = max(depth, h);
+      if (__ldcg(p.excess + v) > 0 && !is_term(p, v)) act++;
+    }
+    if (write_side) p.side[v] = h < p.n ? 1 : 0;
+  });
+  block_add_ll((long long *)&p.ctrl->st_dead, nd);
+  block_add_int(&p.ctrl->aact, act);
+  depth = cg::reduce(cg::tiled_partition<32>(cg::this_thread_block()), depth, cg::greater<int>());
+  if ((threadIdx.x & 31) == 0 && depth > 0) atomicMax(&p.ctrl->adepth, depth);
+}
+
+// Push phase without rounds: every lane polls its vertices' excess and
+// discharges the active ones (the push / relabel rule of discharge()); a vertex
+// of more than 8 arcs is discharged by its whole warp.  As in the rounds, a
+// vertex is only ever discharged by one thread or warp at a time, only its own
+// discharges lower its residuals and excess, and heights only rise, so the
+// races are those of the rounds.  Ends when no vertex is active, or after
+// budget_ns (set by the grid's first thread): the next relabel then gives exact
+// distances again.
+__device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, unsigned long long budget_ns,
+                                              LStats &ls) {
+  Ctrl *c = p.ctrl;
+  const AsyncOwn own = async_own(p.n);
+  const int lane = threadIdx.x & 31;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  unsigned long long t0 = 0;
+  if (lead) {
+    t0 = globaltimer();
+    c->pos_count = 0;
+    c->unexplored = 0;
+  }
+  async_begin(sh);
+  // a dead vertex's parked excess is not polled
+  unsigned live = 0;
+  for (int j = 0; j < own.count; j++) {
+    const int v = own.first + j * own.step + lane;
+    if (v < p.n && !__ldcg(p.dead + v) && !is_term(p, v) && inst_on(p, v)) live |= 1u << j;
+  }
+  TileGroup<32> wg;
+  AsyncIdle st;
+  for (int poll = 0;; poll++) {
+    unsigned have = 0;  // windows in which this lane's vertex holds excess
+    long long ex0 = 0;
+    if (own.count <= 1) {
+      if (live & 1) ex0 = ld_rlx(p.excess + own.first + lane);
+      have = ex0 > 0;
+    } else {
+      long long ex[kAsyncWin];
+#pragma unroll
+      for (int j = 0; j < kAsyncWin; j++)
+        ex[j] = (live >> j) & 1 ? ld_rlx(p.excess + own.first + j * own.step + lane) : 0;
+#pragma unroll
+      for (int j = 0; j < kAsyncWin; j++)
+        if (ex[j] > 0) have |= 1u << j;
+    }
+    bool any = false;
+    if (__any_sync(0xffffffffu, have)) {
+#pragma unroll 1
+      for (int j = 0; j < own.count; j++) {
+        if (!__any_sync(0xffffffffu, (have >> j) & 1)) continue;
+        const int v = own.first + j * own.step + lane;
+        long long x = 0;
+        int h = p.n, beg = 0, deg = 0;
+        if ((have >> j) & 1) {
+          x = own.count <= 1 ? ex0 : __ldcg(p.excess + v);
+          h = __ldcg(p.height + v);
+          beg = __ldg(p.off + v);
+          deg = __ldg(p.off + v + 1) - beg;
+        }
+        const bool act = x > 0 && h < p.n;
+        any |= act;
+        if (act && deg <= kSmallMax) {
+          ls.visits++;
+          discharge_small(p, v, beg, deg, x, h, 0, 0, false, ls);
+        }
+        unsigned wide = __ballot_sync(0xffffffffu, act && deg > kSmallMax);
+        while (wide) {
+          const int src = __ffs(wide) - 1;
+          wide &= wide - 1;
+          discharge(wg, p, __shfl_sync(0xffffffffu, v, src), 0, 0, false, ls, nullptr);
+          __syncwarp();
+        }
+      }
+      any = __any_sync(0xffffffffu, any);
+    }
+    if (lead && (poll & 7) == 0 && globaltimer() - t0 > budget_ns) atomicExch(&c->astop, 1);
+    if (any) {
+      if (threadIdx.x == 0 && (poll & 7) == 0 && ld_rlx(&c->astop)) *(volatile int *)&sh.stop = 1;
+      if (async_busy(sh, st, &c->aidle[1])) break;
+    } else if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) {
+      break;
+    }
+  }
+  sink_flush(p, ls);
+}

@@ -76,6 +76,14 @@ struct Ctrl {
   int dup_at;                   // 1 + an update whose arc an earlier update of the batch names (0: none)
   int nreopen;                  // updates queued for reopening (kept dead set)
   int nrepair;                  // updates queued for the over-capacity repair
+  // barrier-free phases (dmf_async.cuh): blocks idle in the relabel [0] and in
+  // the push phase [1], the push phase's stop word, vertices whose label is not
+  // settled, active vertices and greatest distance of the last relabel
+  int aidle[2];
+  int astop;
+  int aunsettled;
+  int aact;
+  int adepth;
   int pad3;
 };
 

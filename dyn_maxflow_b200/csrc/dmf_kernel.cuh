@@ -49,7 +49,7 @@ enum TraceKind : int {
   TR_CUT_SATURATE = 6, TR_BFS_INIT = 7, TR_BFS_TD = 8, TR_BFS_BU = 9, TR_BFS_FINALIZE = 10, TR_PUSH = 11,
   TR_FLOW = 12, TR_PUSH_HUB = 13, TR_PUSH_HUB_FINISH = 14, TR_PP_INIT = 15, TR_PP_BFS = 16, TR_PP_FINALIZE = 17,
   TR_PP_ROUND = 18, TR_REOPEN = 19, TR_DEAD_SEED = 20, TR_DEAD_PULL = 21, TR_DEAD_CHECK = 23,
-  TR_DEAD_REVIVE = 24
+  TR_DEAD_REVIVE = 24, TR_BFS_ASYNC = 26, TR_PUSH_ASYNC = 27
 };
 
 // Local repair inside a kept dead set: at most this many pull rounds.
@@ -2015,9 +2015,11 @@ __device__ __forceinline__ void ph_pp_round(const Params &p, const Ctrl *sc, int
   }
 }
 
+#include "dmf_async.cuh"
+
 template <int TILE, int BLOCK>
 __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockGroup<BLOCK>::Temp &btmp, int *bci,
-                    long long *bcl, Ctrl *sc) {
+                    long long *bcl, Ctrl *sc, AsyncShared &ash) {
   // c: the control block in global memory (atomics, writes by the lead);
   // sc: this block's copy taken at the last barrier, for every read of a count
   // the previous phase produced
@@ -2211,6 +2213,10 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
   // ---- global relabel / push rounds ---------------------------------------------
   const bool cut_only = p.mode == MODE_CUT;
   const bool topo = p.variant == DMF_VARIANT_TOPO;
+  // Deep graphs: once a relabel has gone kDeepLevels levels, it and the rest of
+  // the solve use the barrier-free phases, where the grid can own every vertex.
+  const bool deep_ok = p.adaptive && p.interval <= kDeepLevels && async_fits(p.n);
+  bool deep = false;
   for (int it = 0;; it++) {
     if (it >= p.max_iters) {
       if (lead) set_err(c, ERR_NO_CONV, it);
@@ -2228,6 +2234,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
     bool bu = false, full = true;
     int L = 0, reached = 0;
     for (;; L++) {
+      if (deep) break;
       const Slot *in = slot_in();
       const int F = in->q + in->hq;
       const long long m_f = in->arcs;
@@ -2235,6 +2242,10 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
       if (F == 0) break;  // complete
       if (!cut_only && P > 0 && reached == P) {
         full = false;  // every active vertex has its exact distance
+        break;
+      }
+      if (deep_ok && L >= kDeepLevels) {
+        deep = true;
         break;
       }
       if (L > 0) m_u -= m_f;
@@ -2250,6 +2261,31 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
       else ph_bfs_td<TILE>(p, in, slot_out(), L, ls);
       if (!next()) return;
       if (lead) c->st_levels++;
+    }
+    if (deep) {
+      const unsigned long long t_bfs = lead ? globaltimer() : 0;
+      for (bool first = true;; first = false) {
+        kind = TR_BFS_ASYNC;
+        items = hubitems = 0;
+        ph_async_bfs(p, ash, L, first, ls);
+        if (!next()) return;
+        ph_async_settled(p, ash);
+        if (!next()) return;
+        if (sc->aunsettled == 0) break;
+      }
+      kind = TR_BFS_FINALIZE;
+      ph_async_finalize(p, want_cut);
+      if (!next()) return;
+      if (lead) c->st_levels += (unsigned long long)max(0, sc->adepth + 1 - L);
+      if (sc->aact == 0 || cut_only) break;
+      // as long again as the relabel took: on the 256 x 256 grid half of that
+      // costs 27 ms a solve, the same 22 ms, twice 24 ms
+      kind = TR_PUSH_ASYNC;
+      items = sc->aact;
+      ph_async_push(p, ash, lead ? globaltimer() - t_bfs : 0, ls);
+      if (!next()) return;
+      if (lead) c->st_rounds++;
+      continue;
     }
     kind = TR_BFS_FINALIZE;
     items = hubitems = 0;
@@ -2297,8 +2333,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_solve(Params p) {
   __shared__ int bci;
   __shared__ long long bcl;
   __shared__ Ctrl snap;
+  __shared__ AsyncShared ash;
   LStats ls;
-  run<TILE, BLOCK>(p, ls, btmp, &bci, &bcl, &snap);
+  run<TILE, BLOCK>(p, ls, btmp, &bci, &bcl, &snap, ash);
   // statistics: one atomic per block and counter
   __syncthreads();
   typedef cub::BlockReduce<unsigned long long, BLOCK> R;

@@ -235,7 +235,8 @@ int dmf_stats_get(const dmf_solver *sv, dmf_stats *st);
  * 10 BFS finalize, 11 push round, 12 flow readout, 13/14 hub push rounds,
  * 15-18 push-pull phase 1, 19 reopen, 20 dead-set pull seeding, 21 pull round,
  * 23 dead-set check, 24 partial revival, 25 capacity claim (duplicate-arc
- * check).  No counterpart in the reference (which
+ * check), 26 barrier-free relabel (deep graphs), 27 barrier-free push phase
+ * (counted as one of dmf_stats.push_rounds).  No counterpart in the reference (which
  * times whole calls with cudaEvents, code/dyn_data_bench.cu:246-258). */
 int dmf_trace_get(dmf_solver *sv, int32_t cap, int32_t *kinds, double *t_us,
                   int32_t *count);
