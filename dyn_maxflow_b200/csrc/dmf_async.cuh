@@ -247,9 +247,9 @@ __device__ __forceinline__ void ph_async_finalize(const Params &p, bool write_si
     }
     if (write_side) p.side[v] = h < p.n ? 1 : 0;
   });
-  block_add_ll((long long *)&p.ctrl->st_dead, nd);
-  block_add_int(&p.ctrl->aact, act);
-  depth = cg::reduce(cg::tiled_partition<32>(cg::this_thread_block()), depth, cg::greater<int>());
+  block_add_ll(0, (long long *)&p.ctrl->st_dead, nd);
+  block_add_int(1, &p.ctrl->aact, act);
+  depth = __reduce_max_sync(0xffffffffu, depth);
   if ((threadIdx.x & 31) == 0 && depth > 0) atomicMax(&p.ctrl->adepth, depth);
 }
 

@@ -8,8 +8,6 @@
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 #include <cooperative_groups/scan.h>
-#include <cub/block/block_reduce.cuh>
-#include <cub/block/block_scan.cuh>
 
 namespace dmfd {
 
@@ -93,6 +91,11 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned atom_add_release_u32(unsigned *p, unsigned x) {
+  unsigned v;
+  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(x) : "memory");
+  return v;
+}
 __device__ __forceinline__ int ld_vol(const int *p) { return *(const volatile int *)p; }
 __device__ __forceinline__ long long ld_vol(const long long *p) { return *(const volatile long long *)p; }
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -102,6 +105,84 @@ __device__ __forceinline__ unsigned long long globaltimer() {
 }
 __device__ __forceinline__ long long atomic_add_ll(long long *p, long long v) {
   return (long long)atomicAdd((unsigned long long *)p, (unsigned long long)v);
+}
+
+// ---- warp-wide sums and prefixes ----------------------------------------------
+// Written out with ballots and redux.sync instead of cooperative_groups'
+// coalesced groups: those find a lane of a partial warp by a software search in
+// every step of a scan, and partial warps are the rule here (a BFS level or a
+// push round of a few hundred vertices).  A phase is bound by the instructions
+// of its slowest warp, so these lengths matter more than the arithmetic.
+__device__ __forceinline__ unsigned lanemask_lt() {
+  unsigned m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+// Sum of v over the lanes of `mask` (every one of them must call it), modulo
+// 2^64: three redux.sync over 24-, 24- and 16-bit pieces, whose 32-lane sums
+// cannot overflow.
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned mask, unsigned long long v) {
+  const unsigned s0 = __reduce_add_sync(mask, (unsigned)v & 0xffffffu);
+  const unsigned s1 = __reduce_add_sync(mask, (unsigned)(v >> 24) & 0xffffffu);
+  const unsigned s2 = __reduce_add_sync(mask, (unsigned)(v >> 48));
+  return (unsigned long long)s0 + ((unsigned long long)s1 << 24) + ((unsigned long long)s2 << 48);
+}
+
+// ---- block accumulators ---------------------------------------------------------
+// Sums that every warp of the grid contributes to in a phase (thousands of
+// same-address atomics would serialise at one L2 slice): warps add into shared
+// memory, and the grid barrier that ends the phase adds a block's totals to
+// global memory before it arrives.  Slot i of a phase has one destination.
+constexpr int kAccSlots = 6;
+struct BlockAcc {
+  unsigned long long v[kAccSlots];
+  unsigned long long *to[kAccSlots];  // bit 0 set: a 32-bit counter
+};
+
+__device__ __forceinline__ BlockAcc &block_acc() {
+  __shared__ BlockAcc acc;
+  return acc;
+}
+
+__device__ __forceinline__ void acc_init() {
+  if (threadIdx.x < kAccSlots) block_acc().v[threadIdx.x] = 0;
+  __syncthreads();
+}
+
+// Whole warps call it (any subset of the block's warps).
+__device__ __forceinline__ void block_add_ll(int slot, long long *p, long long v) {
+  BlockAcc &acc = block_acc();
+  const unsigned long long s = warp_sum_u64(0xffffffffu, (unsigned long long)v);
+  if ((threadIdx.x & 31) == 0 && s) {
+    acc.to[slot] = (unsigned long long *)p;
+    atomicAdd(&acc.v[slot], s);
+  }
+}
+
+__device__ __forceinline__ void block_add_int(int slot, int *p, int v) {
+  BlockAcc &acc = block_acc();
+  const int s = (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
+  if ((threadIdx.x & 31) == 0 && s) {
+    acc.to[slot] = (unsigned long long *)((unsigned long long)p | 1);
+    atomicAdd(&acc.v[slot], (unsigned long long)(long long)s);
+  }
+}
+
+// By lanes of one warp, after a block barrier: adds the totals to their
+// destinations and clears them.
+__device__ __forceinline__ void acc_flush() {
+  BlockAcc &acc = block_acc();
+  const int i = threadIdx.x;
+  if (i < kAccSlots) {
+    const unsigned long long x = acc.v[i];
+    if (x) {
+      const unsigned long long to = (unsigned long long)acc.to[i];
+      if (to & 1) atomicAdd((int *)(to & ~1ull), (int)x);
+      else atomicAdd((unsigned long long *)to, x);
+      acc.v[i] = 0;
+    }
+  }
 }
 
 // ---- bounded grid barrier ---------------------------------------------------
@@ -115,6 +196,11 @@ __device__ __forceinline__ long long atomic_add_ll(long long *p, long long v) {
 // every block, the waiter included.  Polls check the error word and the
 // %globaltimer limit (`limit_ns`, normally kBarrierTimeoutNs) every 64 iterations.
 //
+// The arrival is a release (it orders the block's writes, which the block
+// barrier before it collected), the poll an acquire: no further fence, and no
+// sleep between polls.  With full fences around both and a 32 ns sleep an empty
+// barrier of 296 blocks took 3.1 us; it takes 1.9 us, 0.6 of it the copy below.
+//
 // After the wait, warp 0 copies the whole control block into `snap` (shared
 // memory): the phase that follows reads the counters the previous phase
 // produced from there, so a phase costs G control-block reads instead of one
@@ -124,14 +210,14 @@ __device__ __forceinline__ bool grid_barrier(Ctrl *c, Ctrl *snap, unsigned long 
   __shared__ int s_err;
   __syncthreads();
   if (threadIdx.x < 32) {
+    acc_flush();
+    __syncwarp();
     if (threadIdx.x == 0) {
       const unsigned nb = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
-      __threadfence();
-      const unsigned old = atomicAdd(&c->bar_count, nb);
+      const unsigned old = atom_add_release_u32(&c->bar_count, nb);
       unsigned long long t0 = 0;
       int spins = 0;
       while (((ld_acquire_u32(&c->bar_count) ^ old) & 0x80000000u) == 0) {
-        __nanosleep(32);
         if ((++spins & 63) == 0) {
           if (ld_vol(&c->err)) break;
           const unsigned long long now = globaltimer();
@@ -143,12 +229,16 @@ __device__ __forceinline__ bool grid_barrier(Ctrl *c, Ctrl *snap, unsigned long 
           }
         }
       }
-      __threadfence();
     }
     __syncwarp();
     const int *src = (const int *)c;
     int *dst = (int *)snap;
-    for (int w = threadIdx.x; w < (int)(sizeof(Ctrl) / 4); w += 32) dst[w] = __ldcg(src + w);
+    constexpr int kWords = (int)(sizeof(Ctrl) / 4);
+#pragma unroll
+    for (int i = 0; i < (kWords + 31) / 32; i++) {
+      const int w = threadIdx.x + 32 * i;
+      if (w < kWords) dst[w] = __ldcg(src + w);
+    }
     __syncwarp();
     if (threadIdx.x == 0) s_err = snap->err;
   }
@@ -186,62 +276,41 @@ __device__ __forceinline__ int rot_tiles() { return (int)blockDim.x / 4; }
 __device__ __forceinline__ int rot_threads() { return (int)blockDim.x / 2; }
 
 // ---- queue append (warp-aggregated) -----------------------------------------
-__device__ __forceinline__ void append(int *q, int *tail, int v) {
-  cg::coalesced_group g = cg::coalesced_threads();
+// Position of this thread's entry behind *tail, one atomic for the threads of
+// the warp that call it together.
+__device__ __forceinline__ int reserve_one(int *tail) {
+  const unsigned mask = __activemask(), lt = lanemask_lt();
+  const int leader = __ffs(mask) - 1;
   int base = 0;
-  if (g.thread_rank() == 0) base = atomicAdd(tail, (int)g.size());
-  base = g.shfl(base, 0);
-  q[base + g.thread_rank()] = v;
+  if ((mask & lt) == 0) base = atomicAdd(tail, __popc(mask));
+  return __shfl_sync(mask, base, leader) + __popc(mask & lt);
 }
+
+// Reserves `cnt` (0 to 15) consecutive slots behind *tail for this thread, one
+// atomic for the threads that call it together: the prefix over the lanes is
+// summed bit by bit of the counts.
+__device__ __forceinline__ int reserve(int *tail, int cnt) {
+  const unsigned mask = __activemask(), lt = lanemask_lt();
+  const int leader = __ffs(mask) - 1;
+  int pre = 0, tot = 0;
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    const unsigned m = __ballot_sync(mask, (cnt >> b) & 1);
+    pre += __popc(m & lt) << b;
+    tot += __popc(m) << b;
+  }
+  int base = 0;
+  if ((mask & lt) == 0) base = atomicAdd(tail, tot);
+  return __shfl_sync(mask, base, leader) + pre;
+}
+
+__device__ __forceinline__ void append(int *q, int *tail, int v) { q[reserve_one(tail)] = v; }
 
 // append() into a queue of `cap` entries: *tail still counts every append, so
 // *tail > cap afterwards tells that entries were dropped.
 __device__ __forceinline__ void append_bounded(int *q, int *tail, int v, int cap) {
-  cg::coalesced_group g = cg::coalesced_threads();
-  int base = 0;
-  if (g.thread_rank() == 0) base = atomicAdd(tail, (int)g.size());
-  base = g.shfl(base, 0);
-  if (base + (int)g.thread_rank() < cap) q[base + g.thread_rank()] = v;
-}
-
-__device__ __forceinline__ void agg_add_ll(long long *p, long long v) {
-  cg::coalesced_group g = cg::coalesced_threads();
-  long long s = cg::reduce(g, v, cg::plus<long long>());
-  if (g.thread_rank() == 0 && s) atomic_add_ll(p, s);
-}
-
-__device__ __forceinline__ void agg_add_int(int *p, int v) {
-  cg::coalesced_group g = cg::coalesced_threads();
-  int s = cg::reduce(g, v, cg::plus<int>());
-  if (g.thread_rank() == 0 && s) atomicAdd(p, s);
-}
-
-// Block-wide sum added with one global atomic: for counters that every warp of
-// the grid contributes to at the end of a phase (thousands of same-address
-// atomics otherwise serialise at one L2 slice).  Every thread of the block must
-// call it (uniform control flow: it contains block barriers).
-__device__ __forceinline__ void block_add_ll(long long *p, long long v) {
-  __shared__ long long s_acc;
-  if (threadIdx.x == 0) s_acc = 0;
-  __syncthreads();
-  cg::thread_block_tile<32> w = cg::tiled_partition<32>(cg::this_thread_block());
-  const long long sw = cg::reduce(w, v, cg::plus<long long>());
-  if (w.thread_rank() == 0 && sw) atomicAdd((unsigned long long *)&s_acc, (unsigned long long)sw);
-  __syncthreads();
-  if (threadIdx.x == 0 && s_acc) atomic_add_ll(p, s_acc);
-  __syncthreads();
-}
-
-__device__ __forceinline__ void block_add_int(int *p, int v) {
-  __shared__ int s_acc;
-  if (threadIdx.x == 0) s_acc = 0;
-  __syncthreads();
-  cg::thread_block_tile<32> w = cg::tiled_partition<32>(cg::this_thread_block());
-  const int sw = cg::reduce(w, v, cg::plus<int>());
-  if (w.thread_rank() == 0 && sw) atomicAdd(&s_acc, sw);
-  __syncthreads();
-  if (threadIdx.x == 0 && s_acc) atomicAdd(p, s_acc);
-  __syncthreads();
+  const int at = reserve_one(tail);
+  if (at < cap) q[at] = v;
 }
 
 // ---- groups: one thread, T lanes of a warp, or the whole block ----------------
@@ -269,49 +338,16 @@ struct TileGroup {
     tot = g.shfl(pre + x, T - 1);
     return pre;
   }
-  __device__ __forceinline__ int min_all(int x) { return cg::reduce(g, x, cg::less<int>()); }
-  __device__ __forceinline__ long long sum_all(long long x) { return cg::reduce(g, x, cg::plus<long long>()); }
-  __device__ __forceinline__ bool any(bool x) { return g.any(x); }
-};
-
-template <int BLOCK>
-struct BlockGroup {
-  typedef cub::BlockScan<long long, BLOCK> Scan;
-  typedef cub::BlockReduce<int, BLOCK> RedI;
-  typedef cub::BlockReduce<long long, BLOCK> RedL;
-  union Temp {
-    typename Scan::TempStorage scan;
-    typename RedI::TempStorage redi;
-    typename RedL::TempStorage redl;
-  };
-  Temp &tmp;
-  int *bcast_i;
-  long long *bcast_l;
-  __device__ BlockGroup(Temp &t, int *bi, long long *bl) : tmp(t), bcast_i(bi), bcast_l(bl) {}
-  __device__ __forceinline__ int rank() const { return (int)threadIdx.x; }
-  __host__ __device__ static constexpr int size() { return BLOCK; }
-  __device__ __forceinline__ long long scan(long long x, long long &tot) {
-    long long pre;
-    __syncthreads();
-    Scan(tmp.scan).ExclusiveSum(x, pre, tot);
-    return pre;
-  }
   __device__ __forceinline__ int min_all(int x) {
-    __syncthreads();
-    int r = RedI(tmp.redi).Reduce(x, cub::Min());
-    if (threadIdx.x == 0) *bcast_i = r;
-    __syncthreads();
-    return *bcast_i;
+    if constexpr (T == 32) return __reduce_min_sync(0xffffffffu, x);
+    return cg::reduce(g, x, cg::less<int>());
   }
   __device__ __forceinline__ long long sum_all(long long x) {
-    __syncthreads();
-    long long r = RedL(tmp.redl).Sum(x);
-    if (threadIdx.x == 0) *bcast_l = r;
-    __syncthreads();
-    return *bcast_l;
+    if constexpr (T == 32) return (long long)warp_sum_u64(0xffffffffu, (unsigned long long)x);
+    return cg::reduce(g, x, cg::plus<long long>());
   }
+  __device__ __forceinline__ bool any(bool x) { return g.any(x); }
 };
-
 
 // ---- arc table: (tail, head) -> arc ------------------------------------------
 // Open addressing with linear probing over `nslots` 16-byte slots.  An empty

@@ -227,7 +227,9 @@ __device__ __forceinline__ void ph_saturate(const Params &p) {
       const int beg = __ldg(p.off + s), end = __ldg(p.off + s + 1);
       long long sum = 0;
       for (int a = beg + gt; a < end; a += nt) sum += saturate_arc(p, a);
-      agg_add_ll(p.excess + s, -sum);
+      __syncwarp();
+      sum = (long long)warp_sum_u64(0xffffffffu, (unsigned long long)sum);
+      if ((threadIdx.x & 31) == 0 && sum) atomic_add_ll(p.excess + s, -sum);
     }
     return;
   }
@@ -250,11 +252,17 @@ __device__ __forceinline__ void ph_saturate(const Params &p) {
     const int s = __ldg(p.srcs + lo);
     sum += saturate_arc(p, __ldg(p.off + s) + (j - __ldg(p.src_off + lo)));
   }
-  // threads of a warp that ended on the same source add once
-  cg::coalesced_group g = cg::coalesced_threads();
-  cg::coalesced_group same = cg::labeled_partition(g, cur);
-  sum = cg::reduce(same, sum, cg::plus<long long>());
-  if (same.thread_rank() == 0 && cur >= 0 && sum) atomic_add_ll(p.excess + __ldg(p.srcs + cur), -sum);
+  // a warp that ended on one source adds once
+  __syncwarp();
+  const unsigned on = __ballot_sync(0xffffffffu, cur >= 0);
+  if (!on) return;
+  const int lead = __shfl_sync(0xffffffffu, cur, __ffs(on) - 1);
+  if (__all_sync(0xffffffffu, cur < 0 || cur == lead)) {
+    const long long all = (long long)warp_sum_u64(0xffffffffu, (unsigned long long)sum);
+    if ((threadIdx.x & 31) == 0 && all) atomic_add_ll(p.excess + __ldg(p.srcs + lead), -all);
+  } else if (sum) {
+    atomic_add_ll(p.excess + __ldg(p.srcs + cur), -sum);
+  }
 }
 
 // Arc lookup of OnAdd_kernel (code/dyn_data.h:196-201), which scans the tail's
@@ -703,20 +711,10 @@ __device__ __forceinline__ void ph_bfs_init(const Params &p, Slot *out, bool res
   } else {
     kept = for_live_vertices<4>(p, seed);
   }
-  block_add_int(&c->pos_count, pos);
-  block_add_ll(&c->unexplored, unexpl);
-  block_add_ll(&out->arcs, seed_arcs);
-  if (count_kept) block_add_ll((long long *)&c->st_dead, kept);
-}
-
-// Reserves `cnt` consecutive slots behind *tail for this thread with one atomic
-// per group of threads that call it together.
-__device__ __forceinline__ int reserve(int *tail, int cnt) {
-  cg::coalesced_group g = cg::coalesced_threads();
-  const int pre = cg::exclusive_scan(g, cnt, cg::plus<int>());
-  int base = 0;
-  if (g.thread_rank() == g.size() - 1) base = atomicAdd(tail, pre + cnt);
-  return g.shfl(base, g.size() - 1) + pre;
+  block_add_int(0, &c->pos_count, pos);
+  block_add_ll(1, &c->unexplored, unexpl);
+  block_add_ll(2, &out->arcs, seed_arcs);
+  if (count_kept) block_add_ll(3, (long long *)&c->st_dead, kept);
 }
 
 struct VisitAcc {
@@ -740,8 +738,8 @@ __device__ __forceinline__ void bfs_visit(const Params &p, Slot *out, int nxt, i
 // Counts go to the phase's own slot: a cross-phase counter would be read by a
 // slow block after a fast block already added to it in the next phase.
 __device__ __forceinline__ void flush_visits(const Params &p, Slot *out, VisitAcc &acc) {
-  block_add_ll(&out->arcs, acc.arcs);
-  block_add_int(&out->cnt, acc.reached);
+  block_add_ll(0, &out->arcs, acc.arcs);
+  block_add_int(1, &out->cnt, acc.reached);
 }
 
 // Top-down level (staticMaxFlow_kernel_11, code/dyn_data.h:72-87, run over the
@@ -920,7 +918,7 @@ __device__ __forceinline__ void ph_bfs_finalize(const Params &p, bool full, int 
     }
     if (write_side) p.side[v] = h < p.n ? 1 : 0;
   });
-  block_add_ll((long long *)&p.ctrl->st_dead, nd);
+  block_add_ll(0, (long long *)&p.ctrl->st_dead, nd);
 }
 
 // ---- local repair inside a kept dead set ------------------------------------------
@@ -971,8 +969,8 @@ __device__ __forceinline__ void ph_dead_seed(const Params &p, const Ctrl *sc, Sl
     seeds++;
     need -= ex;
   }
-  block_add_int(&c->dseeds, seeds);
-  block_add_ll(&c->dneed, need);
+  block_add_int(0, &c->dseeds, seeds);
+  block_add_ll(1, &c->dneed, need);
 }
 
 // One pull-relabel round: a warp per deficit of the list, lanes over its arcs.
@@ -1025,7 +1023,7 @@ __device__ __forceinline__ long long pull_excess(const Params &p, cg::thread_blo
       ls.pushes++;
     }
   }
-  return cg::reduce(warp, take, cg::plus<long long>());
+  return (long long)warp_sum_u64(0xffffffffu, (unsigned long long)take);
 }
 
 // Pass 1 on one step: the rest of the deficit moves to dead in-neighbours with
@@ -1053,7 +1051,7 @@ __device__ __forceinline__ long long pull_lower(const Params &p, cg::thread_bloc
     ls.pushes++;
   }
   if (cand > 0 && take < cand) hmin = min(hmin, q.hx);  // still residual
-  return cg::reduce(warp, take, cg::plus<long long>());
+  return (long long)warp_sum_u64(0xffffffffu, (unsigned long long)take);
 }
 
 // Warps first_warp, first_warp + nwarps, ... take the list's deficits; the next
@@ -1124,7 +1122,7 @@ __device__ __forceinline__ void ph_dead_pull(const Params &p, const int *list, i
       if (p.pcur && lane == 0 && stop >= 0) p.pcur[y] = stop - beg;
     }
     if (need > 0) {  // relabel and try again next round (nowhere to go: stays for the check)
-      hmin = cg::reduce(warp, hmin, cg::less<int>());
+      hmin = __reduce_min_sync(0xffffffffu, hmin);
       if (lane == 0 && hmin != INT_MAX) {
         set_dead_label(p, y, hmin + 1);
         ls.relabels++;
@@ -1194,7 +1192,7 @@ __device__ __forceinline__ void ph_dead_check(const Params &p, const Ctrl *sc, S
   } else {
     for_vertices<8>(p, check);
   }
-  block_add_int(&p.ctrl->dleft, left);
+  block_add_int(0, &p.ctrl->dleft, left);
 }
 
 // Partial revival, one level: every dead vertex with a residual arc into the
@@ -1234,8 +1232,8 @@ __device__ __forceinline__ void ph_dead_revive(const Params &p, const Slot *in, 
     const int beg = __ldg(p.off + z), end = __ldg(p.off + z + 1);
     dead_revive_range(p, out, nxt, beg + g.rank(), end, g.size(), ls, scanned, revived);
   });
-  block_add_ll(&out->arcs, scanned);
-  block_add_ll((long long *)&p.ctrl->st_revived, revived);
+  block_add_ll(0, &out->arcs, scanned);
+  block_add_ll(1, (long long *)&p.ctrl->st_revived, revived);
 }
 
 // ---- push rounds ---------------------------------------------------------------
@@ -1265,7 +1263,7 @@ __device__ __forceinline__ long long push_excess(const Params &p, int w, int d, 
 // Every thread of the block calls it at the end of the push phase.
 __device__ __forceinline__ void sink_flush(const Params &p, LStats &ls) {
   if (p.role) return;  // uniform
-  block_add_ll(p.excess + p.t, ls.to_sink);
+  block_add_ll(0, p.excess + p.t, ls.to_sink);
   ls.to_sink = 0;
 }
 
@@ -1606,9 +1604,9 @@ __device__ __forceinline__ RoundIn round_inputs(const Params &p, const Ctrl *c, 
 // Push round, phase 1: non-hub vertices are discharged completely; every hub
 // chunk sums its admissible residual, adds its minimum non-admissible head
 // height to the hub's, and pushes its share of the hub's excess.
-template <int TILE, int BLOCK>
-__device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int r, unsigned round_id, unsigned gepoch, LStats &ls,
-                         typename BlockGroup<BLOCK>::Temp &btmp, int *bci, long long *bcl, bool dph) {
+template <int TILE>
+__device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int r, unsigned round_id, unsigned gepoch,
+                                         LStats &ls, bool dph) {
   Ctrl *c = p.ctrl;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const bool topo = p.variant == DMF_VARIANT_TOPO && !dph;
@@ -1726,7 +1724,7 @@ __device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int
       p, ls, in.nlist, in.nn,
       [&](auto &g, int v) { discharge(g, p, v, r, round_id, !topo, ls, topo ? &seen : nullptr); },
       [&](int v) { return !topo || (__ldcg(p.excess + v) > 0 && inst_on(p, v)); });
-  if (topo) agg_add_int(&c->seen[r % 3], seen);
+  if (topo) block_add_int(1, &c->seen[r % 3], seen);
   sink_flush(p, ls);
 }
 
@@ -1766,16 +1764,16 @@ __device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int
     }
     if (!topo && ex > 0 && h < p.n) enqueue(p, r, round_id, v);
   }
-  if (topo) agg_add_int(&p.ctrl->seen[r % 3], seen);
+  if (topo) block_add_int(0, &p.ctrl->seen[r % 3], seen);
 }
 
 // recalculate_max_flow_kernel_39 (code/dyn_data.h:208-215) as a reduction:
 // flow = excess(t) + sum of negative excess over v != s, t (per instance in
 // batched mode).
-template <int BLOCK>
 // Dead vertices are skipped: a sink or a deficit is a seed of every global
-// relabel, so it is never proven dead.
-__device__ __forceinline__ void ph_flow(const Params &p, typename BlockGroup<BLOCK>::Temp &btmp) {
+// relabel, so it is never proven dead.  The block sums are flushed at the
+// kernel's end.
+__device__ __forceinline__ void ph_flow(const Params &p) {
   long long acc = 0;
   for_live_vertices<8>(p, [&](int v) {
     const long long ex = __ldcg(p.excess + v);
@@ -1788,10 +1786,7 @@ __device__ __forceinline__ void ph_flow(const Params &p, typename BlockGroup<BLO
       acc += c;
     }
   });
-  if (p.inst) return;
-  __syncthreads();
-  long long tot = typename BlockGroup<BLOCK>::RedL(btmp.redl).Sum(acc);
-  if (threadIdx.x == 0 && tot) atomic_add_ll(&p.ctrl->flow, tot);
+  if (!p.inst) block_add_ll(0, &p.ctrl->flow, acc);
 }
 
 __device__ __forceinline__ void clear_slot(Slot *s) {
@@ -1839,7 +1834,7 @@ __device__ __forceinline__ void ph_pp_init(const Params &p, Slot *out) {
     }
     if (pp_active(p, v, ex)) pos++;
   }
-  agg_add_int(&c->pos_count, pos);
+  block_add_int(0, &c->pos_count, pos);
 }
 
 // One level over the frontier: a B vertex x labels B neighbours w with residual
@@ -2017,9 +2012,8 @@ __device__ __forceinline__ void ph_pp_round(const Params &p, const Ctrl *sc, int
 
 #include "dmf_async.cuh"
 
-template <int TILE, int BLOCK>
-__device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockGroup<BLOCK>::Temp &btmp, int *bci,
-                    long long *bcl, Ctrl *sc, AsyncShared &ash) {
+template <int TILE>
+__device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, AsyncShared &ash) {
   // c: the control block in global memory (atomics, writes by the lead);
   // sc: this block's copy taken at the last barrier, for every read of a count
   // the previous phase produced
@@ -2304,7 +2298,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
       kind = TR_PUSH;
       items = in.nn;
       hubitems = in.nh;
-      ph_push1<TILE, BLOCK>(p, in, r, round_id, p.relabel_base + it, ls, btmp, bci, bcl, false);
+      ph_push1<TILE>(p, in, r, round_id, p.relabel_base + it, ls, false);
       if (!next()) return;
       if (in.nh > 0) {
         kind = TR_PUSH_HUB_FINISH;
@@ -2321,7 +2315,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
   }
   kind = TR_FLOW;
   items = hubitems = 0;
-  ph_flow<BLOCK>(p, btmp);
+  ph_flow(p);
   if (lead) c->rounds_used = round_id - p.round_base;
   // the flow phase ends without a barrier; its end is the kernel's end
   if (lead && p.trace && ph + 1 < p.trace_cap) c->trace_len = ph + 1;
@@ -2329,25 +2323,19 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, typename BlockG
 
 template <int TILE, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_solve(Params p) {
-  __shared__ typename BlockGroup<BLOCK>::Temp btmp;
-  __shared__ int bci;
-  __shared__ long long bcl;
   __shared__ Ctrl snap;
   __shared__ AsyncShared ash;
   LStats ls;
-  run<TILE, BLOCK>(p, ls, btmp, &bci, &bcl, &snap, ash);
-  // statistics: one atomic per block and counter
+  acc_init();
+  run<TILE>(p, ls, &snap, ash);
+  // the flow and the statistics: one atomic per block and sum
+  block_add_ll(1, (long long *)&p.ctrl->st_pushes, (long long)ls.pushes);
+  block_add_ll(2, (long long *)&p.ctrl->st_relabels, (long long)ls.relabels);
+  block_add_ll(3, (long long *)&p.ctrl->st_arcs, (long long)(ls.arcs + ls.barcs));
+  block_add_ll(4, (long long *)&p.ctrl->st_visits, (long long)ls.visits);
+  block_add_ll(5, (long long *)&p.ctrl->st_barcs, (long long)ls.barcs);
   __syncthreads();
-  typedef cub::BlockReduce<unsigned long long, BLOCK> R;
-  __shared__ typename R::TempStorage rt;
-  unsigned long long v[5] = {ls.pushes, ls.relabels, ls.arcs + ls.barcs, ls.visits, ls.barcs};
-  unsigned long long *dst[5] = {&p.ctrl->st_pushes, &p.ctrl->st_relabels, &p.ctrl->st_arcs, &p.ctrl->st_visits,
-                                &p.ctrl->st_barcs};
-  for (int i = 0; i < 5; i++) {
-    unsigned long long s = R(rt).Sum(v[i]);
-    if (threadIdx.x == 0 && s) atomicAdd(dst[i], s);
-    __syncthreads();
-  }
+  if (threadIdx.x < 32) acc_flush();
 }
 
 
