@@ -233,9 +233,9 @@ __device__ __forceinline__ void ph_async_settled(const Params &p, AsyncShared &s
 
 // ph_bfs_finalize of a complete relabel, which also counts the active vertices
 // and finds the greatest distance.
-__device__ __forceinline__ void ph_async_finalize(const Params &p, bool write_side) {
+__device__ __forceinline__ void ph_async_finalize(const Params &p, bool write_side, bool listed) {
   int nd = 0, act = 0, depth = 0;
-  for_live_vertices<4>(p, [&](int v) {
+  for_live<4>(p, listed, [&](int v) {
     const int h = __ldcg(p.height + v);
     if (h == UNV) {
       p.dead[v] = 1;

@@ -65,14 +65,14 @@ struct Ctrl {
   // deficits found among them, and those left after the local repair
   int dcand;
   int dseeds;
-  long long dneed;
   int dleft;
   int dkept;                    // 1: the dead set was kept for the global relabels
   unsigned long long st_barcs;  // adjacency entries read by global-relabel BFS levels
   unsigned long long st_dseeds; // deficits inside the kept dead set (first local pass)
   unsigned long long st_revived; // dead vertices revived because they reach a deficit left over
   int dup_at;                   // 1 + an update whose arc an earlier update of the batch names (0: none)
-  int nreopen;                  // updates queued for reopening (kept dead set)
+  int berr, berr_info;          // error bits of a batch's lookup, and the update
+  int nreopen;                  // updates queued for saturation: source arcs, reopened arcs
   int nrepair;                  // updates queued for the over-capacity repair
   // barrier-free phases (dmf_async.cuh): blocks idle in the relabel [0] and in
   // the push phase [1], the push phase's stop word, vertices whose label is not

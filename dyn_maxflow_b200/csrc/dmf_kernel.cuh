@@ -75,6 +75,13 @@ struct Params {
   int *fq[2], *wq[2], *aq;     // non-hub vertex queues
   int *dq;                     // dead vertices whose excess the batch changed (kept dead set)
   int *dlab;                   // distance from excess inside the dead set, (wave << 4) | level
+  // Live vertices of the solver: lq[0 .. *lst) holds every live vertex (and
+  // vertices that died since the list was built), each once; inl marks them.
+  // Built by every solve that starts from a revived dead set, added to by the
+  // partial revival.  Null: no list (allocation-free solve).
+  int *lq, *lst;
+  unsigned char *inl;
+  int nact;                    // vertices of the instances this call works on
   int *pcur;                   // per vertex: where in its row its last pull found enough (long rows; may be null)
   int2 *fh[2], *wh[2], *ah;    // hub chunk queues
   const int2 *hch;             // every hub's chunks (bottom-up BFS, topology-driven rounds)
@@ -166,6 +173,12 @@ __device__ __forceinline__ bool inst_on(const Params &p, int v) {
 
 __device__ __forceinline__ void set_err(Ctrl *c, int bit, int info) {
   if (atomicOr(&c->err, bit) == 0) c->err_info = info;
+}
+
+// The same for an error in a batch's updates: the batch is rejected after the
+// barrier, with what it claimed undone.
+__device__ __forceinline__ void set_batch_err(Ctrl *c, int bit, int info) {
+  if (atomicOr(&c->berr, bit) == 0) c->berr_info = info;
 }
 
 // A dead vertex whose excess a batch lowers joins the candidate list once
@@ -273,17 +286,57 @@ __device__ __forceinline__ void ph_saturate(const Params &p) {
 // the tail's adjacency, and the line is only read.  Equal (tail, head) pairs
 // in a CSR with duplicate arcs resolve to the last arc among them, as
 // OnAdd_kernel's scan keeps the last match.  The lookup validates vertex ids,
-// capacities and arcs; an arc named twice is found by the claim (ph_claim).
+// capacities and arcs; an arc named twice is found by the claim.
 
-// Updates a thread looks up side by side: their probes are in flight together.
-constexpr int kLookupBatch = 4;
+// Updates a thread looks up side by side: their probes are in flight together
+// (four spill and cost 5% at R-MAT 22).
+constexpr int kLookupBatch = 2;
 
-__device__ __forceinline__ void ph_lookup(const Params &p) {
+// Whether an update of u->v that leaves residual on the arc has to be saturated
+// at once: an arc out of a source (every solve keeps those saturated: nothing
+// is pushed into a source), or, with the dead set kept, one from a dead tail to
+// a live head (ph_reopen).
+__device__ __forceinline__ bool saturates(const Params &p, int u, int v) {
+  const bool du = p.keep_dead && __ldcg(p.dead + u), dv = p.keep_dead && __ldcg(p.dead + v);
+  return !is_src(p, v) && (is_src(p, u) || (du && !dv));
+}
+
+// What follows the swap of an update's capacity word: `old` is the word it got
+// back.  Moves the residual by the difference; an arc whose residual went
+// negative carries more flow than its new capacity and is queued for the repair
+// (ph_repair) rather than repaired here, so that a rejected batch only has to
+// undo additions; one with residual left is queued when `sat`.
+__device__ __forceinline__ void claimed(const Params &p, int i, int e, int w, unsigned long long old, bool residual,
+                                        bool sat) {
+  if ((unsigned)(old >> 32) == (unsigned)p.epoch) {  // named twice: this update changes nothing
+    p.uold[i] = -1;
+    atomicCAS(&p.ctrl->dup_at, 0, i + 1);
+    return;
+  }
+  const int oc = (int)(unsigned)old;
+  p.uold[i] = oc;
+  const int delta = w - oc;
+  if (!residual || !delta) return;
+  const int r = atomicAdd(p.res + e, delta) + delta;
+  if (r < 0) append_bounded(p.wq[0], &p.ctrl->nrepair, i, p.n + 1);
+  else if (r > 0 && sat) append_bounded(p.aq, &p.ctrl->nreopen, i, p.n + 1);
+}
+
+// Lookup, and in the same pass (caps_bounded) the claim and the capacity apply
+// of OnAdd_kernel (code/dyn_data.h:202-205): the new capacity goes in, the
+// residual moves by the difference.  In recompute mode only the capacity
+// changes (update_kernel, code/dyn_data_bench.cu:300-322).  One pass instead of
+// two spares a barrier and the second read of the batch: whole 1% batches take
+// 95 -> 90 us at R-MAT 18, 131 -> 121 at R-MAT 20; at R-MAT 22 and 24 (230 and
+// 640 us), where random DRAM accesses set the time, the two ways are equal.  A graph with capacities
+// above kMaxUpdateCap has to compare an update with its partner's capacity
+// before the batch, so there the claim waits for the barrier (ph_claim_apply).
+__device__ __forceinline__ void ph_lookup(const Params &p, bool residual) {
   const int nt = gridDim.x * blockDim.x, gt = spread_thread();
   for (int i0 = gt; i0 < p.k; i0 += kLookupBatch * nt) {
     int u[kLookupBatch], v[kLookupBatch], w[kLookupBatch], e[kLookupBatch];
     long long slot[kLookupBatch];
-    bool on[kLookupBatch], pend[kLookupBatch];
+    bool on[kLookupBatch], pend[kLookupBatch], sat[kLookupBatch];
 #pragma unroll
     for (int j = 0; j < kLookupBatch; j++) {
       const int i = i0 + j * nt;
@@ -295,16 +348,12 @@ __device__ __forceinline__ void ph_lookup(const Params &p) {
 #pragma unroll
     for (int j = 0; j < kLookupBatch; j++) {
       e[j] = -1;
-      pend[j] = false;
+      pend[j] = sat[j] = false;
       if (!on[j]) continue;
       const int i = i0 + j * nt;
-      p.uarc[i] = -1;
       if (u[j] < 0 || u[j] >= p.n || v[j] < 0 || v[j] >= p.n || w[j] < 0 || w[j] > kMaxUpdateCap) {
-        set_err(p.ctrl, ERR_BAD_UPDATE, i);
-        on[j] = false;
-      } else if (u[j] == v[j]) {
-        on[j] = false;  // ignored, as OnAdd_kernel does (code/dyn_data.h:194)
-      } else {
+        set_batch_err(p.ctrl, ERR_BAD_UPDATE, i);
+      } else if (u[j] != v[j]) {  // equal: ignored, as OnAdd_kernel does (code/dyn_data.h:194)
         slot[j] = arc_slot0(u[j], v[j], p.nslots);
         pend[j] = true;
       }
@@ -316,6 +365,11 @@ __device__ __forceinline__ void ph_lookup(const Params &p) {
 #pragma unroll
       for (int j = 0; j < kLookupBatch; j++)
         if (pend[j]) s[j] = load_slot(p.atab + slot[j]);
+      if (probe == 0 && residual) {  // in flight beside the first slots
+#pragma unroll
+        for (int j = 0; j < kLookupBatch; j++)
+          if (pend[j]) sat[j] = saturates(p, u[j], v[j]);
+      }
       bool any = false;
 #pragma unroll
       for (int j = 0; j < kLookupBatch; j++) {
@@ -324,6 +378,7 @@ __device__ __forceinline__ void ph_lookup(const Params &p) {
           e[j] = s[j].arc;
           pend[j] = false;
         } else if (s[j].tail == kEmptyTail) {
+          set_batch_err(p.ctrl, ERR_UNKNOWN_ARC, i0 + j * nt);
           pend[j] = false;
         } else {
           slot[j] = slot[j] + 1 == p.nslots ? 0 : slot[j] + 1;
@@ -332,64 +387,41 @@ __device__ __forceinline__ void ph_lookup(const Params &p) {
       }
       if (!any) break;
     }
+    unsigned long long old[kLookupBatch];
 #pragma unroll
     for (int j = 0; j < kLookupBatch; j++) {
       if (!on[j]) continue;
       const int i = i0 + j * nt;
-      if (e[j] < 0) {
-        set_err(p.ctrl, ERR_UNKNOWN_ARC, i);
-        continue;
-      }
-      if (!p.caps_bounded && (long long)w[j] + cap_of(p, __ldg(p.par + e[j])) > INT_MAX) {
-        set_err(p.ctrl, ERR_BAD_UPDATE, i);
-        continue;
+      if (p.caps_bounded) {
+        if (e[j] >= 0) old[j] = atomicExch(p.capx + e[j], cap_word(p, w[j]));
+      } else if (e[j] >= 0 && (long long)w[j] + cap_of(p, __ldg(p.par + e[j])) > INT_MAX) {
+        set_batch_err(p.ctrl, ERR_BAD_UPDATE, i);
+        e[j] = -1;
       }
       p.uarc[i] = e[j];
     }
+    if (!p.caps_bounded) continue;
+#pragma unroll
+    for (int j = 0; j < kLookupBatch; j++)
+      if (e[j] >= 0) claimed(p, i0 + j * nt, e[j], w[j], old[j], residual, sat[j]);
   }
 }
 
-// Claim and capacity apply of OnAdd_kernel (code/dyn_data.h:202-205) in one
-// pass: the new capacity goes in, the residual moves by the difference.  An
-// arc whose residual went negative carries more flow than its new capacity;
-// it is queued for the repair (ph_repair) rather than repaired here, so that a
-// rejected batch only has to undo additions.  With the dead set kept, an arc
-// from a dead tail to a live head that has residual now is queued for
-// reopening.  In recompute mode only the capacity changes (update_kernel,
-// code/dyn_data_bench.cu:300-322).
+// The claim and the capacity apply by themselves (capacities not bounded).
 __device__ __forceinline__ void ph_claim_apply(const Params &p, bool residual) {
   const int nt = gridDim.x * blockDim.x, gt = spread_thread();
-  const unsigned ep = (unsigned)p.epoch;
   for (int i = gt; i < p.k; i += nt) {
     const int e = __ldcg(p.uarc + i);
     if (e < 0) continue;
     const int w = __ldg(p.uw + i);
-    bool du = false, dv = false;
-    int u = 0, v = 0;
-    if (residual && p.keep_dead) {
-      u = __ldg(p.usrc + i);
-      v = __ldg(p.udst + i);  // the lookup matched adj[e] == udst[i]
-      du = __ldcg(p.dead + u) != 0;
-      dv = __ldcg(p.dead + v) != 0;
-    }
-    const unsigned long long old = atomicExch(p.capx + e, cap_word(p, w));
-    if ((unsigned)(old >> 32) == ep) {  // named twice: this update changes nothing
-      p.uold[i] = -1;
-      atomicCAS(&p.ctrl->dup_at, 0, i + 1);
-      continue;
-    }
-    const int oc = (int)(unsigned)old;
-    p.uold[i] = oc;
-    const int delta = w - oc;
-    if (!residual || !delta) continue;
-    const int r = atomicAdd(p.res + e, delta) + delta;
-    if (r < 0) append_bounded(p.wq[0], &p.ctrl->nrepair, i, p.n + 1);
-    else if (r > 0 && du && !dv && !is_src(p, v)) append_bounded(p.aq, &p.ctrl->nreopen, i, p.n + 1);
+    const bool sat = residual && saturates(p, __ldg(p.usrc + i), __ldg(p.udst + i));
+    claimed(p, i, e, w, atomicExch(p.capx + e, cap_word(p, w)), residual, sat);
   }
 }
 
 // A rejected batch: every update that changed its arc (the first to name it)
-// puts the capacity and the residual back.
+// puts the capacity and the residual back.  A thread walks the updates that it
+// claimed itself (the same numbering as ph_lookup and ph_claim_apply).
 __device__ __forceinline__ void ph_unclaim(const Params &p, bool residual) {
   const int nt = gridDim.x * blockDim.x, gt = spread_thread();
   for (int i = gt; i < p.k; i += nt) {
@@ -445,18 +477,20 @@ __device__ __forceinline__ void reopen_update(const Params &p, int i) {
   const int e = __ldcg(p.uarc + i);
   if (e < 0) return;
   const int u = __ldg(p.usrc + i), v = __ldg(p.udst + i);  // adj[e] == udst[i]
-  if (!__ldcg(p.dead + u) || __ldcg(p.dead + v) || is_src(p, v)) return;
+  if (!saturates(p, u, v)) return;
   const int r = __ldcg(p.res + e);
   if (r <= 0) return;
   p.res[e] = 0;
   atomicAdd(p.res + __ldg(p.par + e), r);
   atomic_add_ll(p.excess + u, -(long long)r);
   atomic_add_ll(p.excess + v, (long long)r);
-  add_dead_cand(p, u);
+  if (!is_src(p, u)) add_dead_cand(p, u);
 }
 
-// The apply queued the updates that can need it (dead tail, live head,
-// residual left); past the queue's capacity every update is looked at.
+// The apply queued the updates that can need it (source arcs; dead tail, live
+// head; residual left); past the queue's capacity every update is looked at.
+// The source arcs among the updates are the only ones a batch can leave
+// unsaturated, so a batch never sweeps a source's row.
 __device__ __forceinline__ void ph_reopen(const Params &p, const Ctrl *sc) {
   const int nt = gridDim.x * blockDim.x, gt = spread_thread();
   const int nq = sc->nreopen;
@@ -597,8 +631,8 @@ __device__ __forceinline__ void for_vertices(const Params &p, F &&f) {
   }
 }
 
-// Every live vertex of the call, f(v); returns how many dead vertices this
-// thread passed over.  A warp takes windows of 512 vertices and first reads
+// Every live vertex of the call by a sweep, f(v); returns how many this thread
+// saw.  A warp takes windows of 512 vertices and first reads
 // their dead flags as one 16-byte load per lane: a window with no live vertex
 // (nearly all of them when a batch keeps the dead set) costs that load and a
 // vote.  Other windows are walked like for_vertices (v = window + 32 j + lane,
@@ -608,13 +642,14 @@ constexpr int kWindow = 512;
 
 template <int U, class F>
 __device__ __forceinline__ int for_live_vertices(const Params &p, F &&f) {
-  int dead_seen = 0;
+  int seen = 0;
   if (p.inst_active) {
     for_vertices<U>(p, [&](int v, bool is_dead) {
-      if (is_dead) dead_seen++;
-      else f(v);
+      if (is_dead) return;
+      seen++;
+      f(v);
     });
-    return dead_seen;
+    return seen;
   }
   const int lane = threadIdx.x & 31;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -632,10 +667,7 @@ __device__ __forceinline__ int for_live_vertices(const Params &p, F &&f) {
       all_dead = true;
       for (int i = 0; i < mine; i++) all_dead &= __ldcg(p.dead + b + i) != 0;
     }
-    if (__all_sync(0xffffffffu, all_dead)) {
-      dead_seen += mine;
-      continue;
-    }
+    if (__all_sync(0xffffffffu, all_dead)) continue;
     for (int j0 = 0; j0 < kWindow / 32; j0 += U) {
       unsigned char dd[U];
 #pragma unroll
@@ -646,13 +678,45 @@ __device__ __forceinline__ int for_live_vertices(const Params &p, F &&f) {
 #pragma unroll
       for (int j = 0; j < U; j++) {
         const long long v = w0 + (j0 + j) * 32 + lane;
-        if (v >= p.n) continue;
-        if (dd[j]) dead_seen++;
-        else f((int)v);
+        if (v >= p.n || dd[j]) continue;
+        seen++;
+        f((int)v);
       }
     }
   }
-  return dead_seen;
+  return seen;
+}
+
+// Every live vertex of the call, f(v); returns how many this thread saw.  A
+// batch that keeps the dead set (`listed`) walks the live list while that is
+// short; entries that died since are skipped by their flag.  With ~400 live
+// vertices of 1 M the walk takes one dependent load more than an empty phase
+// where the sweep reads every flag (seed pass 9 -> 4 us at R-MAT 20, 16 -> 4 at
+// R-MAT 22); past a quarter of the vertices the sweep's coalesced reads win.
+template <int U, class F>
+__device__ __forceinline__ int for_live(const Params &p, bool listed, F &&f) {
+  if (listed) {
+    const int cnt = __ldcg(p.lst);
+    if (4ll * cnt < p.n) {
+      const int nt = gridDim.x * blockDim.x;
+      int seen = 0;
+      for (int i = spread_thread(); i < cnt; i += nt) {
+        const int v = __ldcg(p.lq + i);
+        if (__ldcg(p.dead + v) || !inst_on(p, v)) continue;
+        seen++;
+        f(v);
+      }
+      return seen;
+    }
+  }
+  return for_live_vertices<U>(p, f);
+}
+
+// A vertex that a batch revived joins the live list (claimed by this thread).
+__device__ __forceinline__ void list_revived(const Params &p, int v) {
+  if (__ldcg(p.inl + v)) return;  // died after the list was built, still listed
+  p.inl[v] = 1;
+  append(p.lq, p.lst, v);
 }
 
 // Seeds (my_init_1, code/dyn_data.h:60-67): t and every deficit vertex other
@@ -662,15 +726,17 @@ __device__ __forceinline__ int for_live_vertices(const Params &p, F &&f) {
 // statistic (first relabel of a batch that kept them).  Vertices of instances
 // outside the call's mask are not touched at all: their labels and dead set
 // stay as their own last solve left them.
-__device__ __forceinline__ void ph_bfs_init(const Params &p, Slot *out, bool reset_dead, bool count_kept) {
+__device__ __forceinline__ void ph_bfs_init(const Params &p, Slot *out, bool reset_dead, bool count_kept,
+                                            bool listed) {
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   Ctrl *c = p.ctrl;
   if (gt == 0) {
     c->act_q = 0;
     c->act_hq = 0;
     c->wtail[0] = c->whtail[0] = c->seen[0] = 0;  // written by push round 0
+    if (reset_dead && p.lst) *p.lst = 0;          // rebuilt by the flow readout
   }
-  int pos = 0, kept = 0;
+  int pos = 0, live = 0;
   long long unexpl = 0, seed_arcs = 0;
   auto seed = [&](int v) {
     long long ex = __ldcg(p.excess + v);
@@ -709,12 +775,12 @@ __device__ __forceinline__ void ph_bfs_init(const Params &p, Slot *out, bool res
       seed(v);
     });
   } else {
-    kept = for_live_vertices<4>(p, seed);
+    live = for_live<4>(p, listed, seed);
   }
   block_add_int(0, &c->pos_count, pos);
   block_add_ll(1, &c->unexplored, unexpl);
   block_add_ll(2, &out->arcs, seed_arcs);
-  if (count_kept) block_add_ll(3, (long long *)&c->st_dead, kept);
+  if (count_kept) block_add_ll(3, (long long *)&c->st_dead, (long long)(gt == 0 ? p.nact : 0) - live);
 }
 
 struct VisitAcc {
@@ -903,9 +969,10 @@ __device__ __forceinline__ void ph_bfs_bu(const Params &p, Slot *out, int L, LSt
 // early-stopped BFS gives them the valid lower bound `floor`.
 // Vertices already dead are skipped: they sit at height V and side 0 since the
 // BFS that proved them dead.
-__device__ __forceinline__ void ph_bfs_finalize(const Params &p, bool full, int floor_h, bool write_side) {
+__device__ __forceinline__ void ph_bfs_finalize(const Params &p, bool full, int floor_h, bool write_side,
+                                                bool listed) {
   int nd = 0;
-  for_live_vertices<8>(p, [&](int v) {
+  for_live<8>(p, listed, [&](int v) {
     const int h = __ldcg(p.height + v);
     if (h == UNV) {
       if (full) {
@@ -958,7 +1025,6 @@ __device__ __forceinline__ void ph_dead_seed(const Params &p, const Ctrl *sc, Sl
   const int nt = gridDim.x * blockDim.x, gt = spread_thread();
   Ctrl *c = p.ctrl;
   int seeds = 0;
-  long long need = 0;
   const int nc = min(sc->dcand, p.n + 1);
   for (int i = gt; i < nc; i += nt) {
     const int v = __ldcg(p.dq + i);
@@ -967,10 +1033,8 @@ __device__ __forceinline__ void ph_dead_seed(const Params &p, const Ctrl *sc, Sl
     set_dead_label(p, v, 1);
     append(p.fq[0], &out->q, v);
     seeds++;
-    need -= ex;
   }
   block_add_int(0, &c->dseeds, seeds);
-  block_add_ll(1, &c->dneed, need);
 }
 
 // One pull-relabel round: a warp per deficit of the list, lanes over its arcs.
@@ -1055,10 +1119,13 @@ __device__ __forceinline__ long long pull_lower(const Params &p, cg::thread_bloc
 }
 
 // Warps first_warp, first_warp + nwarps, ... take the list's deficits; the next
-// round's list is appended behind *ntail.
+// round's list is appended behind *ntail.  seed: the list is the candidates
+// themselves (a list of at most a candidate per warp spares the seed phase);
+// the deficits among them are labelled 1 and counted here.
 __device__ __forceinline__ void ph_dead_pull(const Params &p, const int *list, int nn, int *nxt, int *ntail,
-                                             int first_warp, int nwarps, unsigned round_id, LStats &ls) {
+                                             int first_warp, int nwarps, unsigned round_id, bool seed, LStats &ls) {
   const int lane = threadIdx.x & 31;
+  int seeds = 0;
   cg::thread_block_tile<32> warp = cg::tiled_partition<32>(cg::this_thread_block());
   for (int i = first_warp; i < nn; i += nwarps) {
     int y = 0;
@@ -1069,9 +1136,13 @@ __device__ __forceinline__ void ph_dead_pull(const Params &p, const int *list, i
     }
     y = warp.shfl(y, 0);
     need = warp.shfl(need, 0);
-    if (need <= 0) continue;
+    if (need <= 0 || (seed && is_term(p, y))) continue;
     ItemTimer tm(p);
-    const int hy = dead_label(p, y);
+    const int hy = seed ? 1 : dead_label(p, y);
+    if (seed && lane == 0) {
+      set_dead_label(p, y, 1);
+      seeds++;
+    }
     const int beg = __ldg(p.off + y), end = __ldg(p.off + y + 1);
     long long got = 0;
     int hmin = INT_MAX;  // lowest label over the dead in-neighbours still residual
@@ -1132,6 +1203,7 @@ __device__ __forceinline__ void ph_dead_pull(const Params &p, const int *list, i
     if (lane == 0 && got) atomic_add_ll(p.excess + y, got);
     tm.done(ls, y);
   }
+  if (seed) block_add_int(0, &p.ctrl->dseeds, seeds);
 }
 
 // Pull rounds from round r0 on, in the calling block alone, once the list is
@@ -1145,14 +1217,15 @@ constexpr int kPullTail = 64;
 // revives it.
 constexpr int kPullTailRounds = 6;
 
-__device__ __forceinline__ void pull_tail_rounds(const Params &p, int r0, int nn, unsigned round_base, LStats &ls) {
+__device__ __forceinline__ void pull_tail_rounds(const Params &p, int r0, const int *first, int nn, bool seed,
+                                                 unsigned round_base, LStats &ls) {
   __shared__ int s_tail;
   const int r_end = min(kDeadRounds, r0 + kPullTailRounds);
   for (int r = r0; r < r_end && nn > 0; r++) {
     if (threadIdx.x == 0) s_tail = 0;
     __syncthreads();
-    ph_dead_pull(p, p.fq[r & 1], nn, p.fq[(r + 1) & 1], &s_tail, threadIdx.x >> 5, blockDim.x >> 5,
-                 round_base + (unsigned)(r - r0) + 1, ls);
+    ph_dead_pull(p, r == r0 ? first : p.fq[r & 1], nn, p.fq[(r + 1) & 1], &s_tail, threadIdx.x >> 5, blockDim.x >> 5,
+                 round_base + (unsigned)(r - r0) + 1, seed && r == r0, ls);
     __syncthreads();
     nn = s_tail;
     __syncthreads();
@@ -1178,6 +1251,7 @@ __device__ __forceinline__ void ph_dead_check(const Params &p, const Ctrl *sc, S
     if (is_dead && !is_term(p, v) && __ldcg(p.excess + v) < 0 && revive_claim(p, v)) {
       left++;
       p.dead[v] = 0;
+      list_revived(p, v);
       if (deg_of(p, v) > p.hub_deg) append_hub(p, p.fh[0], &out->hq, v);
       else append(p.fq[0], &out->q, v);
     }
@@ -1209,6 +1283,7 @@ __device__ __forceinline__ void dead_revive_range(const Params &p, Slot *out, in
     if (__ldcg(p.res + __ldg(p.par + a)) <= 0 || !__ldcg(p.dead + x) || is_term(p, x)) continue;
     if (!revive_claim(p, x)) continue;
     p.dead[x] = 0;
+    list_revived(p, x);
     revived++;
     if (deg_of(p, x) > p.hub_deg) append_hub(p, p.fh[nxt], &out->hq, x);
     else append(p.fq[nxt], &out->q, x);
@@ -1771,11 +1846,13 @@ __device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int
 // flow = excess(t) + sum of negative excess over v != s, t (per instance in
 // batched mode).
 // Dead vertices are skipped: a sink or a deficit is a seed of every global
-// relabel, so it is never proven dead.  The block sums are flushed at the
-// kernel's end.
-__device__ __forceinline__ void ph_flow(const Params &p) {
+// relabel, so it is never proven dead.  A solve that started from a revived
+// dead set sweeps every flag and builds the live list on the way (all
+// instances, also those the call left alone).  The block sums are flushed at
+// the kernel's end.
+__device__ __forceinline__ void ph_flow(const Params &p, bool listed) {
   long long acc = 0;
-  for_live_vertices<8>(p, [&](int v) {
+  auto add = [&](int v) {
     const long long ex = __ldcg(p.excess + v);
     long long c = 0;
     if (is_snk(p, v)) c = ex;
@@ -1785,7 +1862,38 @@ __device__ __forceinline__ void ph_flow(const Params &p) {
     } else {
       acc += c;
     }
-  });
+  };
+  if (listed || !p.lst) {
+    for_live<8>(p, listed, add);
+  } else {
+    const int lane = threadIdx.x & 31;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long w0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWindow; w0 < p.n;
+         w0 += nw * kWindow) {
+      const long long b = w0 + 16 * lane;
+      bool all_dead = true;
+      if (b + 16 <= p.n) {
+        const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(p.dead + b));
+        constexpr unsigned one = 0x01010101u;
+        *reinterpret_cast<uint4 *>(p.inl + b) = make_uint4(x.x ^ one, x.y ^ one, x.z ^ one, x.w ^ one);
+        all_dead = (x.x & x.y & x.z & x.w) == one;
+      } else {
+        for (long long v = b; v < p.n; v++) {
+          const bool d = __ldcg(p.dead + v) != 0;
+          p.inl[v] = d ? 0 : 1;
+          all_dead &= d;
+        }
+      }
+      if (__all_sync(0xffffffffu, all_dead)) continue;
+#pragma unroll 4
+      for (int j = 0; j < kWindow / 32; j++) {
+        const long long v = w0 + 32 * j + lane;
+        if (v >= p.n || __ldcg(p.dead + v)) continue;
+        append(p.lq, p.lst, (int)v);
+        if (inst_on(p, (int)v)) add((int)v);
+      }
+    }
+  }
   if (!p.inst) block_add_ll(0, &p.ctrl->flow, acc);
 }
 
@@ -2066,31 +2174,38 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   } else if (p.mode == MODE_DYNAMIC || p.mode == MODE_RECOMPUTE) {
     const bool dyn = p.mode == MODE_DYNAMIC;
     kind = TR_LOOKUP;
-    ph_lookup(p);
-    if (!next()) return;
-    kind = TR_APPLY;
-    ph_claim_apply(p, dyn);
-    if (!next()) return;
-    if (sc->dup_at) {  // every claim is done: undo them, reject the batch
-      ph_unclaim(p, dyn);
-      if (lead) set_err(c, ERR_DUP_ARC, sc->dup_at - 1);
+    ph_lookup(p, dyn);
+    if (!next()) {  // the wait ran out: every thread takes back its own claims
+      if (p.caps_bounded) ph_unclaim(p, dyn);
+      return;
+    }
+    if (!p.caps_bounded && !sc->berr) {
+      kind = TR_APPLY;
+      ph_claim_apply(p, dyn);
+      if (!next()) return;
+    }
+    if (sc->berr || sc->dup_at) {  // every claim is done: undo them, reject the batch
+      if (p.caps_bounded || !sc->berr) ph_unclaim(p, dyn);
+      if (lead) set_err(c, sc->berr ? sc->berr : ERR_DUP_ARC, sc->berr ? sc->berr_info : sc->dup_at - 1);
       return;
     }
     if (dyn) {
-      kind = TR_REPAIR;
-      ph_repair(p, sc);
-      if (!next()) return;
+      // most small batches leave nothing over capacity and nothing to saturate
+      if (sc->nrepair) {
+        kind = TR_REPAIR;
+        ph_repair(p, sc);
+        if (!next()) return;
+      }
       if (p.variant == DMF_VARIANT_PP && !p.keep_dead) {  // with the dead set kept, ph_reopen does it
         kind = TR_CUT_SATURATE;
         ph_cut_saturate(p);
         if (!next()) return;
       }
-      // source saturation and reopening touch disjoint arcs (a reopened arc's
-      // tail is dead, so neither it nor its partner is a source arc): one phase
-      kind = TR_SATURATE;
-      ph_saturate(p);
-      if (p.keep_dead) ph_reopen(p, sc);
-      if (!next()) return;
+      if (sc->nreopen) {
+        kind = TR_REOPEN;
+        ph_reopen(p, sc);
+        if (!next()) return;
+      }
     } else {
       kind = TR_INIT_RES;
       ph_init_res(p);
@@ -2107,33 +2222,40 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   bool revive = true;  // the first global relabel revives every vertex
   if (p.mode == MODE_DYNAMIC && p.keep_dead) {
     revive = false;
-    kind = TR_DEAD_SEED;
-    items = sc->dcand;
-    hubitems = 0;
-    ph_dead_seed(p, sc, slot_out());
-    if (!next()) return;
-    if (lead) c->st_dseeds = (unsigned long long)sc->dseeds;
-    if (sc->dseeds > 0) {
-      const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int ncand = min(sc->dcand, p.n + 1);
+    const bool direct = ncand <= nwarps;  // the first round finds the deficits among the candidates itself
+    if (ncand > 0 && !direct) {
+      kind = TR_DEAD_SEED;
+      items = ncand;
+      hubitems = 0;
+      ph_dead_seed(p, sc, slot_out());
+      if (!next()) return;
+    }
+    if (ncand > 0) {
       for (int r = 0; r < kDeadRounds; r++) {
-        const Slot *in = slot_in();
-        if (in->q == 0) break;
+        const bool seed = direct && r == 0;
+        const int *list = seed ? p.dq : p.fq[r & 1];
+        const int cnt = seed ? ncand : slot_in()->q;
+        if (cnt == 0) break;
         kind = TR_DEAD_PULL;
-        items = in->q;
+        items = cnt;
         hubitems = 0;
-        if (in->q <= kPullTail) {  // the remaining rounds in one block
-          if (blockIdx.x == 0) pull_tail_rounds(p, r, in->q, round_id, ls);
+        if (cnt <= kPullTail) {  // the remaining rounds in one block
+          if (blockIdx.x == 0) pull_tail_rounds(p, r, list, cnt, seed, round_id, ls);
           round_id += (unsigned)(kDeadRounds - r);
           if (!next()) return;
           if (lead) c->rounds_used = round_id - p.round_base;
           break;
         }
         round_id++;
-        ph_dead_pull(p, p.fq[r & 1], in->q, p.fq[(r + 1) & 1], &slot_out()->q, spread_group<32>(), nwarps, round_id,
-                     ls);
+        ph_dead_pull(p, list, cnt, p.fq[(r + 1) & 1], &slot_out()->q, spread_group<32>(), nwarps, round_id, seed, ls);
         if (!next()) return;
         if (lead) c->rounds_used = round_id - p.round_base;
       }
+      if (lead) c->st_dseeds = (unsigned long long)sc->dseeds;
+    }
+    if (sc->dseeds > 0) {
       kind = TR_DEAD_CHECK;
       items = sc->dcand;
       hubitems = 0;
@@ -2206,6 +2328,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
 
   // ---- global relabel / push rounds ---------------------------------------------
   const bool cut_only = p.mode == MODE_CUT;
+  const bool listed = !revive && p.lst;  // the live list holds for this solve
   const bool topo = p.variant == DMF_VARIANT_TOPO;
   // Deep graphs: once a relabel has gone kDeepLevels levels, it and the rest of
   // the solve use the barrier-free phases, where the grid can own every vertex.
@@ -2218,7 +2341,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     }
     kind = TR_BFS_INIT;
     items = hubitems = 0;
-    ph_bfs_init(p, slot_out(), it == 0 && revive, it == 0 && !revive);
+    ph_bfs_init(p, slot_out(), it == 0 && revive, it == 0 && !revive, listed);
     if (!next()) return;
     if (lead) c->st_outer++;
     const int P = sc->pos_count;
@@ -2268,7 +2391,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
         if (sc->aunsettled == 0) break;
       }
       kind = TR_BFS_FINALIZE;
-      ph_async_finalize(p, want_cut);
+      ph_async_finalize(p, want_cut, listed);
       if (!next()) return;
       if (lead) c->st_levels += (unsigned long long)max(0, sc->adepth + 1 - L);
       if (sc->aact == 0 || cut_only) break;
@@ -2283,7 +2406,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     }
     kind = TR_BFS_FINALIZE;
     items = hubitems = 0;
-    ph_bfs_finalize(p, full, L + 1, full && want_cut);
+    ph_bfs_finalize(p, full, L + 1, full && want_cut, listed);
     if (!next()) return;
     const int A = sc->act_q + sc->act_hq;
     if (A == 0 || cut_only) break;
@@ -2315,7 +2438,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   }
   kind = TR_FLOW;
   items = hubitems = 0;
-  ph_flow(p);
+  ph_flow(p, listed);
   if (lead) c->rounds_used = round_id - p.round_base;
   // the flow phase ends without a barrier; its end is the kernel's end
   if (lead && p.trace && ph + 1 < p.trace_cap) c->trace_len = ph + 1;

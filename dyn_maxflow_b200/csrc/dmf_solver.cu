@@ -160,6 +160,8 @@ struct dmf_solver {
   unsigned char *dead = nullptr, *side = nullptr;
   int *dlab = nullptr;    // dead-set repair labels, tagged with the launch epoch
   int *pcur = nullptr;    // per vertex: pull scan cursor in its row
+  int *lq = nullptr, *lst = nullptr;  // live vertices of the solved state, and their count
+  unsigned char *inl = nullptr;       // per vertex: in the live list
   bool caps_bounded = false;  // every capacity <= 2^30 - 1 (updates keep it so)
   int *qbuf = nullptr;    // 6 vertex queues (frontier x2, worklist x2, active, dead-set candidates)
   int2 *hqbuf = nullptr;  // 5 hub-chunk queues, same roles
@@ -355,6 +357,15 @@ Params make_params(dmf_solver *sv, int mode, int k, const int *d_src, const int 
   p.dq = sv->qbuf + 5 * N;
   p.dlab = sv->dlab;
   p.pcur = sv->pcur;
+  p.lq = sv->lq;
+  p.lst = sv->lst;
+  p.inl = sv->inl;
+  p.nact = sv->n;
+  if (sv->use_active) {
+    p.nact = 0;
+    for (int i = 0; i < sv->ninst; i++)
+      if (sv->h_inst_active[i]) p.nact += sv->vbase[i + 1] - sv->vbase[i];
+  }
   p.ah = sv->hqbuf + 4 * NC;
   p.hch = sv->hch;
   p.nhch = sv->nchunk;
@@ -732,6 +743,8 @@ int dmf_static_maxflow_noalloc(int32_t n, int32_t m, const int32_t *d_index, con
     p.dq = nullptr;  // static solves never keep a dead set
     p.dlab = nullptr;
     p.pcur = nullptr;
+    p.lq = p.lst = nullptr;
+    p.inl = nullptr;
     // no hubs in this mode (hub_deg = INT_MAX): the hub structures are never read
     int2 *hub_dummy = (int2 *)carve(kNoAllocAlign);
     long long *ll_dummy = (long long *)carve(kNoAllocAlign);
@@ -876,7 +889,8 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
       (st = dalloc(sv, &sv->atab, (size_t)arc_table_slots((long long)M))) || (st = dalloc(sv, &sv->capx, M)) ||
       (st = dalloc(sv, &sv->res, M)) || (st = dalloc(sv, &sv->height, N)) || (st = dalloc(sv, &sv->stamp, N)) ||
       (st = dalloc(sv, &sv->excess, N)) || (st = dalloc(sv, &sv->dead, N)) || (st = dalloc(sv, &sv->side, N)) ||
-      (st = dalloc(sv, &sv->qbuf, 6 * N)) || (st = dalloc(sv, &sv->dlab, N)) || (st = dalloc(sv, &sv->pcur, N)) || (st = dalloc(sv, &sv->ctrl, 1)))
+      (st = dalloc(sv, &sv->qbuf, 6 * N)) || (st = dalloc(sv, &sv->dlab, N)) || (st = dalloc(sv, &sv->pcur, N)) || (st = dalloc(sv, &sv->lq, N)) ||
+      (st = dalloc(sv, &sv->lst, 1)) || (st = dalloc(sv, &sv->inl, N)) || (st = dalloc(sv, &sv->ctrl, 1)))
     return st;
   std::vector<int2> hub_chunks;
   std::vector<int> hub_base(g->n, -1);
@@ -933,6 +947,8 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->dlab, 0, 4 * N, S);
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->pcur, 0, 4 * N, S);
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->side, 0, N, S);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sv->inl, 0, N, S);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sv->lst, 0, 4, S);
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->excess, 0, 8 * N, S);
   if (e == cudaSuccess) e = cudaMallocHost(&sv->h_ctrl, sizeof(Ctrl));
   if (e == cudaSuccess) e = cudaEventCreate(&sv->ev0);
@@ -980,7 +996,7 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
 
 int64_t dmf::solver_footprint(int64_t n, int64_t m) {
   // adj, par, res, capacity words; the arc table; off, labels, stamps,
-  // excess, marks, repair labels, hub bases and six vertex queues (rounded up)
+  // excess, marks, repair labels, hub bases, the live list and six vertex queues (rounded up)
   return 20 * m + (int64_t)sizeof(ArcSlot) * arc_table_slots(m) + 64 * n;
 }
 
@@ -1513,6 +1529,9 @@ int dmf_solver_copy_state(dmf_solver *dst, const dmf_solver *src) {
     CK(cudaMemcpyAsync(dst->stamp, src->stamp, 4 * N, cudaMemcpyDeviceToDevice, S), "D2D stamp");
     CK(cudaMemcpyAsync(dst->dead, src->dead, N, cudaMemcpyDeviceToDevice, S), "D2D dead");
     CK(cudaMemcpyAsync(dst->side, src->side, N, cudaMemcpyDeviceToDevice, S), "D2D side");
+    CK(cudaMemcpyAsync(dst->lq, src->lq, 4 * N, cudaMemcpyDeviceToDevice, S), "D2D live list");
+    CK(cudaMemcpyAsync(dst->lst, src->lst, 4, cudaMemcpyDeviceToDevice, S), "D2D live list");
+    CK(cudaMemcpyAsync(dst->inl, src->inl, N, cudaMemcpyDeviceToDevice, S), "D2D live list");
     CK(cudaMemcpyAsync(dst->chunk_mark, src->chunk_mark, 8 * NC, cudaMemcpyDeviceToDevice, S), "D2D marks");
     CK(cudaMemcpyAsync(dst->chunk_tmin, src->chunk_tmin, 4 * NC, cudaMemcpyDeviceToDevice, S), "D2D marks");
     CK(cudaStreamSynchronize(S), "copy state");
