@@ -86,7 +86,7 @@ _sig("dmf_gen_batches", C.c_int, VP, C.c_int32, C.c_double, C.c_double, C.c_doub
      C.c_int32, C.c_int32, C.c_uint64, PP, PP, PP, PP)
 _sig("dmf_solver_create", C.c_int, VP, C.c_int32, C.c_int32, C.POINTER(Opts), VP, PP)
 _sig("dmf_static_maxflow", C.c_int, VP, C.POINTER(C.c_int64))
-_sig("dmf_apply_updates", C.c_int, VP, C.c_int32, I32P, I32P, I32P, C.POINTER(C.c_int64))
+_sig("dmf_apply_updates", C.c_int, VP, C.c_int32, VP, VP, VP, C.POINTER(C.c_int64))
 _sig("dmf_apply_updates_device", C.c_int, VP, C.c_int32, VP, VP, VP, C.POINTER(C.c_int64))
 _sig("dmf_recompute", C.c_int, VP, C.c_int32, I32P, I32P, I32P, C.POINTER(C.c_int64))
 _sig("dmf_recompute_device", C.c_int, VP, C.c_int32, VP, VP, VP, C.POINTER(C.c_int64))
@@ -162,6 +162,8 @@ def _check(st: int) -> None:
 def _i32(a) -> np.ndarray:
     """Contiguous int32 view or copy; values that int32 cannot hold exactly
     (out of range, fractional) raise instead of wrapping to another id."""
+    if type(a) is np.ndarray and a.dtype == np.int32 and a.flags.c_contiguous:
+        return a
     a = np.asarray(a)
     if a.dtype != np.int32 and a.size:
         if a.dtype.kind not in "biuf":
@@ -337,7 +339,7 @@ class Solver:
     def apply_updates(self, src, dst, w) -> int:
         src, dst, w = _i32(src), _i32(dst), _i32(w)
         f = C.c_int64()
-        _check(_L.dmf_apply_updates(self._h, len(src), src, dst, w, C.byref(f)))
+        _check(_L.dmf_apply_updates(self._h, len(src), src.ctypes.data, dst.ctypes.data, w.ctypes.data, C.byref(f)))
         return f.value
 
     def apply_updates_device(self, d_src: int, d_dst: int, d_w: int, k: int) -> int:

@@ -38,7 +38,8 @@ struct Slot {
   int pad;
 };
 
-// Control block of one solver (device memory, cleared before every launch).
+// Control block of one solver (device memory, zero between launches: the last
+// block of a launch clears it).
 struct Ctrl {
   unsigned int bar_count;     // grid barrier: arrivals (low bits) and generation (top bit)
   unsigned int bar_gen;       // unused
@@ -82,7 +83,14 @@ struct Ctrl {
   int aunsettled;
   int aact;
   int adepth;
-  int pad3;
+  unsigned done;                // blocks that have ended
+};
+
+// Where a launch leaves its result in pinned host memory: the control block,
+// then the launch's number.
+struct HostResult {
+  Ctrl c;
+  unsigned seq;
 };
 
 // ---- memory helpers ---------------------------------------------------------
@@ -95,6 +103,14 @@ __device__ __forceinline__ unsigned atom_add_release_u32(unsigned *p, unsigned x
   unsigned v;
   asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(x) : "memory");
   return v;
+}
+__device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned *p, unsigned x) {
+  unsigned v;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(x) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_sys_u32(unsigned *p, unsigned x) {
+  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
 }
 __device__ __forceinline__ int ld_vol(const int *p) { return *(const volatile int *)p; }
 __device__ __forceinline__ long long ld_vol(const long long *p) { return *(const volatile long long *)p; }
@@ -269,6 +285,9 @@ __device__ __forceinline__ int spread_group(int rot = 0) {
   const int t = (int)threadIdx.x - rot;
   return ((t < 0 ? t + (int)blockDim.x : t) / T) * gridDim.x + blockIdx.x;
 }
+// Threads numbered warps first over the blocks: lanes keep consecutive numbers
+// (coalesced reads of a batch's arrays), warps 0 .. G-1 sit in G blocks.
+__device__ __forceinline__ int spread_lane() { return spread_group<32>() * 32 + (int)(threadIdx.x & 31); }
 // Rotations used by the phases: hub chunks from warp 0, tile items from the
 // first warp of the second quarter of the block, one-thread items from the
 // middle.

@@ -101,6 +101,17 @@ struct Params {
   unsigned relabel_base;
   const int *usrc, *udst, *uw;
   int k;
+  // A short host batch is read where it lies in pinned host memory (xsrc, ...)
+  // and the lookup leaves a device copy in ucopy (usrc, udst, uw) for the phases
+  // after it.  Else xsrc == usrc, ... and ucopy is null.
+  const int *xsrc, *xdst, *xw;
+  int *ucopy;
+  int ustride;
+  // Result in pinned host memory (null: the host copies the control block).
+  HostResult *hres;
+  long long *hflow;  // per-instance flows
+  unsigned seq;      // the launch's number
+  int ninst;
   // Several independent instances in one residual graph (batched mode): role
   // bit 0 = a source, bit 1 = a sink, inst = instance of each vertex, flows per
   // instance.  Single instance: role == nullptr, s and t above.
@@ -332,7 +343,7 @@ __device__ __forceinline__ void claimed(const Params &p, int i, int e, int w, un
 // above kMaxUpdateCap has to compare an update with its partner's capacity
 // before the batch, so there the claim waits for the barrier (ph_claim_apply).
 __device__ __forceinline__ void ph_lookup(const Params &p, bool residual) {
-  const int nt = gridDim.x * blockDim.x, gt = spread_thread();
+  const int nt = gridDim.x * blockDim.x, gt = spread_lane();
   for (int i0 = gt; i0 < p.k; i0 += kLookupBatch * nt) {
     int u[kLookupBatch], v[kLookupBatch], w[kLookupBatch], e[kLookupBatch];
     long long slot[kLookupBatch];
@@ -341,9 +352,19 @@ __device__ __forceinline__ void ph_lookup(const Params &p, bool residual) {
     for (int j = 0; j < kLookupBatch; j++) {
       const int i = i0 + j * nt;
       on[j] = i < p.k;
-      u[j] = on[j] ? __ldg(p.usrc + i) : 0;
-      v[j] = on[j] ? __ldg(p.udst + i) : 0;
-      w[j] = on[j] ? __ldg(p.uw + i) : 0;
+      u[j] = on[j] ? __ldcg(p.xsrc + i) : 0;
+      v[j] = on[j] ? __ldcg(p.xdst + i) : 0;
+      w[j] = on[j] ? __ldcg(p.xw + i) : 0;
+    }
+    if (p.ucopy) {
+#pragma unroll
+      for (int j = 0; j < kLookupBatch; j++) {
+        const int i = i0 + j * nt;
+        if (!on[j]) continue;
+        p.ucopy[i] = u[j];
+        p.ucopy[p.ustride + i] = v[j];
+        p.ucopy[2 * p.ustride + i] = w[j];
+      }
     }
 #pragma unroll
     for (int j = 0; j < kLookupBatch; j++) {
@@ -409,12 +430,12 @@ __device__ __forceinline__ void ph_lookup(const Params &p, bool residual) {
 
 // The claim and the capacity apply by themselves (capacities not bounded).
 __device__ __forceinline__ void ph_claim_apply(const Params &p, bool residual) {
-  const int nt = gridDim.x * blockDim.x, gt = spread_thread();
+  const int nt = gridDim.x * blockDim.x, gt = spread_lane();
   for (int i = gt; i < p.k; i += nt) {
     const int e = __ldcg(p.uarc + i);
     if (e < 0) continue;
-    const int w = __ldg(p.uw + i);
-    const bool sat = residual && saturates(p, __ldg(p.usrc + i), __ldg(p.udst + i));
+    const int w = __ldcg(p.uw + i);
+    const bool sat = residual && saturates(p, __ldcg(p.usrc + i), __ldcg(p.udst + i));
     claimed(p, i, e, w, atomicExch(p.capx + e, cap_word(p, w)), residual, sat);
   }
 }
@@ -423,14 +444,14 @@ __device__ __forceinline__ void ph_claim_apply(const Params &p, bool residual) {
 // puts the capacity and the residual back.  A thread walks the updates that it
 // claimed itself (the same numbering as ph_lookup and ph_claim_apply).
 __device__ __forceinline__ void ph_unclaim(const Params &p, bool residual) {
-  const int nt = gridDim.x * blockDim.x, gt = spread_thread();
+  const int nt = gridDim.x * blockDim.x, gt = spread_lane();
   for (int i = gt; i < p.k; i += nt) {
     const int e = __ldcg(p.uarc + i);
     if (e < 0) continue;
     const int oc = __ldcg(p.uold + i);
     if (oc < 0) continue;
     p.capx[e] = (unsigned long long)(unsigned)oc;
-    const int delta = __ldg(p.uw + i) - oc;
+    const int delta = __ldcg(p.uw + i) - oc;
     if (residual && delta) atomicSub(p.res + e, delta);
   }
 }
@@ -448,7 +469,7 @@ __device__ __forceinline__ void repair_update(const Params &p, int i) {
   if (r >= 0) return;
   atomicAdd(p.res + e, -r);
   atomicAdd(p.res + __ldg(p.par + e), r);
-  const int u = __ldg(p.usrc + i), v = __ldg(p.udst + i);
+  const int u = __ldcg(p.usrc + i), v = __ldcg(p.udst + i);
   atomic_add_ll(p.excess + u, -(long long)r);
   atomic_add_ll(p.excess + v, (long long)r);
   if (p.keep_dead) {  // the overflow returns to the tail: excess that can cover the head's deficit
@@ -476,7 +497,7 @@ __device__ __forceinline__ void ph_repair(const Params &p, const Ctrl *sc) {
 __device__ __forceinline__ void reopen_update(const Params &p, int i) {
   const int e = __ldcg(p.uarc + i);
   if (e < 0) return;
-  const int u = __ldg(p.usrc + i), v = __ldg(p.udst + i);  // adj[e] == udst[i]
+  const int u = __ldcg(p.usrc + i), v = __ldcg(p.udst + i);  // adj[e] == udst[i]
   if (!saturates(p, u, v)) return;
   const int r = __ldcg(p.res + e);
   if (r <= 0) return;
@@ -509,7 +530,7 @@ __device__ __forceinline__ void ph_cut_saturate(const Params &p) {
   for (int i = gt; i < p.k; i += nt) {
     int e = __ldcg(p.uarc + i);
     if (e < 0) continue;
-    int u = __ldg(p.usrc + i), v = __ldg(p.udst + i);  // adj[e] == udst[i]
+    int u = __ldcg(p.usrc + i), v = __ldcg(p.udst + i);  // adj[e] == udst[i]
     if (is_term(p, u) || is_term(p, v)) continue;
     if (p.side[u] == 0 && p.side[v] == 1) {
       int r = __ldcg(p.res + e);
@@ -2444,6 +2465,34 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   if (lead && p.trace && ph + 1 < p.trace_cap) c->trace_len = ph + 1;
 }
 
+// The last block to end writes the control block and the per-instance flows to
+// pinned host memory, clears both for the next launch, and then sets the
+// launch's number, which the host polls: no memset before a launch and no copy
+// after it (each a separate engine operation of 2-4 us).
+__device__ __forceinline__ void publish(const Params &p) {
+  if (!p.hres) return;
+  __shared__ int s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atom_add_acqrel_u32(&p.ctrl->done, 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  int *c = (int *)p.ctrl;
+  volatile int *h = (volatile int *)&p.hres->c;
+  for (int w = threadIdx.x; w < (int)(sizeof(Ctrl) / 4); w += blockDim.x) {
+    h[w] = __ldcg(c + w);
+    c[w] = 0;
+  }
+  if (p.inst) {
+    for (int i = threadIdx.x; i < p.ninst; i += blockDim.x) {
+      *(volatile long long *)(p.hflow + i) = __ldcg(p.inst_flow + i);
+      p.inst_flow[i] = 0;
+    }
+  }
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) st_release_sys_u32(&p.hres->seq, p.seq);
+}
+
 template <int TILE, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_solve(Params p) {
   __shared__ Ctrl snap;
@@ -2459,6 +2508,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_solve(Params p) {
   block_add_ll(5, (long long *)&p.ctrl->st_barcs, (long long)ls.barcs);
   __syncthreads();
   if (threadIdx.x < 32) acc_flush();
+  publish(p);
 }
 
 

@@ -194,7 +194,10 @@ struct dmf_solver {
   int *h_ubuf = nullptr;  // pinned host staging
   int h_kcap = 0;
   Ctrl *ctrl = nullptr;
-  Ctrl *h_ctrl = nullptr;  // pinned
+  HostResult *h_res = nullptr;  // pinned: what the last launch left
+  unsigned seq = 0;             // number of the last launch
+  bool direct = false;          // the staged batch is read from pinned host memory
+  bool ms_pending = false;      // st.last_ms is not read from the events yet
   unsigned long long *trace = nullptr;  // device timeline (opts.flags & DMF_FLAG_TRACE)
   int trace_cap = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -243,7 +246,7 @@ void free_all(dmf_solver *sv) {
   for (void *q : sv->allocs) cudaFree(q);
   sv->allocs.clear();
   if (sv->h_ubuf) cudaFreeHost(sv->h_ubuf);
-  if (sv->h_ctrl) cudaFreeHost(sv->h_ctrl);
+  if (sv->h_res) cudaFreeHost(sv->h_res);
   if (sv->h_inst_flow) cudaFreeHost(sv->h_inst_flow);
   sv->h_inst_flow = nullptr;
   if (sv->h_inst_active) cudaFreeHost(sv->h_inst_active);
@@ -253,7 +256,7 @@ void free_all(dmf_solver *sv) {
   if (sv->ev0) cudaEventDestroy(sv->ev0);
   if (sv->ev1) cudaEventDestroy(sv->ev1);
   sv->h_ubuf = nullptr;
-  sv->h_ctrl = nullptr;
+  sv->h_res = nullptr;
   sv->ev0 = sv->ev1 = nullptr;
 }
 
@@ -314,7 +317,7 @@ int ensure_host_ubuf(dmf_solver *sv, int k) {
   if (k <= sv->h_kcap) return DMF_OK;
   int want = std::max(k, 1024);
   int *nb = nullptr;
-  CK(cudaMallocHost(&nb, sizeof(int) * 3 * (size_t)want), "cudaMallocHost");
+  CK(cudaHostAlloc((void **)&nb, sizeof(int) * 3 * (size_t)want, cudaHostAllocMapped), "cudaHostAlloc");
   if (sv->h_ubuf) {
     cudaStreamSynchronize(sv->stream);
     cudaFreeHost(sv->h_ubuf);
@@ -384,10 +387,25 @@ Params make_params(dmf_solver *sv, int mode, int k, const int *d_src, const int 
   p.chunk_mark = sv->chunk_mark;
   p.chunk_tmin = sv->chunk_tmin;
   p.relabel_base = sv->relabel_base;
-  p.usrc = d_src;
-  p.udst = d_dst;
-  p.uw = d_w;
+  p.usrc = p.xsrc = d_src;
+  p.udst = p.xdst = d_dst;
+  p.uw = p.xw = d_w;
+  p.ucopy = nullptr;
+  p.ustride = 0;
+  if (sv->direct && d_src == sv->ubuf) {
+    const size_t HK = (size_t)sv->h_kcap;
+    p.xsrc = sv->h_ubuf;
+    p.xdst = sv->h_ubuf + HK;
+    p.xw = sv->h_ubuf + 2 * HK;
+    p.ucopy = sv->ubuf;
+    p.ustride = sv->kcap;
+  }
   p.k = k;
+  p.hres = sv->h_res;
+  p.hflow = sv->h_inst_flow;
+  p.ninst = sv->ninst;
+  if (++sv->seq == 0) sv->seq = 1;
+  p.seq = sv->seq;
   p.ctrl = sv->ctrl;
   p.mode = mode;
   p.variant = sv->opts.variant;
@@ -417,27 +435,48 @@ Params make_params(dmf_solver *sv, int mode, int k, const int *d_src, const int 
 
 int launch(dmf_solver *sv, int mode, int k, const int *d_src, const int *d_dst, const int *d_w) {
   Params p = make_params(sv, mode, k, d_src, d_dst, d_w);
-  CK(cudaMemsetAsync(sv->ctrl, 0, sizeof(Ctrl), sv->stream), "memset ctrl");
-  if (sv->inst_flow) CK(cudaMemsetAsync(sv->inst_flow, 0, 8 * (size_t)sv->ninst, sv->stream), "memset flows");
   void *args[] = {&p};
   CK(cudaLaunchCooperativeKernel((const void *)pick_kernel(sv->tile, sv->minb), dim3(sv->grid), dim3(sv->block), args, 0,
                                  sv->stream),
      "cooperative launch");
-  CK(cudaMemcpyAsync(sv->h_ctrl, sv->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, sv->stream), "D2H ctrl");
-  if (sv->inst_flow)
-    CK(cudaMemcpyAsync(sv->h_inst_flow, sv->inst_flow, 8 * (size_t)sv->ninst, cudaMemcpyDeviceToHost, sv->stream),
-       "D2H flows");
   return DMF_OK;
+}
+
+// Waits until the launch's result is in pinned memory: polls its number there
+// (a few us less than an event wait), and the event now and then, so that a
+// launch that failed ends the wait too.
+int wait_result(dmf_solver *sv) {
+  for (unsigned spin = 1;; spin++) {
+    if (__atomic_load_n(&sv->h_res->seq, __ATOMIC_ACQUIRE) == sv->seq) return DMF_OK;
+    if (spin % 4096 == 0) {
+      const cudaError_t q = cudaEventQuery(sv->ev1);
+      if (q == cudaSuccess) {
+        if (__atomic_load_n(&sv->h_res->seq, __ATOMIC_ACQUIRE) == sv->seq) return DMF_OK;
+        return fail(DMF_ERR_CUDA, "the solve kernel left no result");
+      }
+      if (q != cudaErrorNotReady) return cuda_fail(q, "solve");
+    }
+    __builtin_ia32_pause();
+  }
+}
+
+// Device time of the last call, read from its events when somebody asks.
+void resolve_ms(const dmf_solver *csv) {
+  dmf_solver *sv = const_cast<dmf_solver *>(csv);
+  if (!sv->ms_pending) return;
+  sv->ms_pending = false;
+  float ms = 0;
+  if (cudaSetDevice(sv->dev) == cudaSuccess && cudaEventSynchronize(sv->ev1) == cudaSuccess &&
+      cudaEventElapsedTime(&ms, sv->ev0, sv->ev1) == cudaSuccess)
+    sv->st.last_ms = ms;
 }
 
 // Waits for the launch sequence, records timing and maps device errors.
 int finish(dmf_solver *sv, int64_t *flow, bool need_cut_valid) {
   CK(cudaEventRecord(sv->ev1, sv->stream), "event record");
-  CK(cudaEventSynchronize(sv->ev1), "solve");
-  float ms = 0;
-  cudaEventElapsedTime(&ms, sv->ev0, sv->ev1);
-  const Ctrl &c = *sv->h_ctrl;
-  sv->st.last_ms = ms;
+  if (int st = wait_result(sv)) return st;
+  const Ctrl &c = sv->h_res->c;
+  sv->ms_pending = true;
   sv->st.outer_iters = (int64_t)c.st_outer;
   sv->st.bfs_levels = (int64_t)c.st_levels;
   sv->st.push_rounds = (int64_t)c.st_rounds;
@@ -512,23 +551,41 @@ int check_updates_args(dmf_solver *sv, int32_t k, const void *a, const void *b, 
   return DMF_OK;
 }
 
-// Host batch -> pinned staging -> device, pipelined: the three arrays are cut
-// into pieces of kStagePiece updates; copier threads fill the pinned buffer
-// piece by piece (piece i by thread i mod kStageCopiers, so early pieces finish
-// first) while one issuer thread starts the H2D of each piece as soon as it is
-// in, so the copy engine works while later pieces are still being copied.  A
-// batch of fewer than four pieces is copied and sent whole.
-constexpr size_t kStagePiece = 1 << 18;  // updates (1 MiB of int32)
+// Host batch -> pinned staging -> device.  Up to kDirectUpdates updates are not
+// copied to the device at all: the lookup reads them once, coalesced, from the
+// pinned buffer, which several threads fill when the batch is not small (1,000
+// updates at R-MAT 20: 53 us a call against 68 with three copies; 32,000: 70
+// against 95; 256,000: 231 against 385).  Larger batches are pipelined: the three arrays are cut into pieces of an eighth of the batch,
+// within [kPieceMin, kPieceMax]; copier threads fill the pinned buffer piece by
+// piece (piece i by thread i mod kStageCopiers, so early pieces finish first)
+// while one issuer thread starts the H2D of each piece as soon as it is in, so
+// the copy engine works while later pieces are still being copied.
+constexpr size_t kDirectUpdates = 1 << 18;
+constexpr size_t kCopyAlone = 1 << 14;  // batches up to this size are copied by the calling thread
+constexpr size_t kPieceMin = 1 << 15, kPieceMax = 1 << 18;  // updates (128 KiB, 1 MiB of int32)
 constexpr int kStageCopiers = 8;
 
-int stage_batch(dmf_solver *sv, int32_t k, const int32_t *src, const int32_t *dst, const int32_t *w) {
+int stage_batch(dmf_solver *sv, int32_t k, const int32_t *src, const int32_t *dst, const int32_t *w, bool direct_ok) {
   int st;
   CK(cudaSetDevice(sv->dev), "cudaSetDevice");
   if ((st = ensure_ubuf(sv, k)) || (st = ensure_host_ubuf(sv, k))) return st;
   const size_t K = (size_t)sv->kcap, HK = (size_t)sv->h_kcap, n = (size_t)k;
   const int32_t *from[3] = {src, dst, w};
-  const size_t per = (n + kStagePiece - 1) / kStagePiece, total = 3 * per;
-  if (total < 4) {
+  const size_t cut = std::min(kPieceMax, std::max(kPieceMin, n / 8));
+  const size_t per = (n + cut - 1) / cut, total = 3 * per;
+  sv->direct = direct_ok && n <= kDirectUpdates;
+  if (sv->direct) {
+    if (n <= kCopyAlone) {
+      for (int a = 0; a < 3 && n > 0; a++) std::memcpy(sv->h_ubuf + a * HK, from[a], 4 * n);
+    } else {
+#pragma omp parallel num_threads(kStageCopiers)
+      {
+        const size_t tid = (size_t)omp_get_thread_num(), nthr = (size_t)omp_get_num_threads();
+        const size_t b = n * tid / nthr, e = n * (tid + 1) / nthr;
+        for (int a = 0; a < 3; a++) std::memcpy(sv->h_ubuf + a * HK + b, from[a] + b, 4 * (e - b));
+      }
+    }
+  } else if (per < 2) {
     for (int a = 0; a < 3 && n > 0; a++) {
       std::memcpy(sv->h_ubuf + a * HK, from[a], 4 * n);
       CK(cudaMemcpyAsync(sv->ubuf + a * K, sv->h_ubuf + a * HK, 4 * n, cudaMemcpyHostToDevice, sv->stream),
@@ -540,8 +597,8 @@ int stage_batch(dmf_solver *sv, int32_t k, const int32_t *src, const int32_t *ds
     cudaError_t err = cudaSuccess;
     auto piece = [&](size_t i, size_t &a, size_t &b, size_t &e) {
       a = i / per;
-      b = (i % per) * kStagePiece;
-      e = std::min(n, b + kStagePiece);
+      b = (i % per) * cut;
+      e = std::min(n, b + cut);
     };
 #pragma omp parallel num_threads(kStageCopiers + 1)
     {
@@ -577,7 +634,7 @@ int host_updates(dmf_solver *sv, int mode, int32_t k, const int32_t *src, const 
   int st = check_updates_args(sv, k, src, dst, w);
   if (st) return st;
   if (mode == MODE_DYNAMIC && !sv->solved) return fail(DMF_ERR_NOT_SOLVED, "apply_updates before a solve");
-  if ((st = stage_batch(sv, k, src, dst, w))) return st;
+  if ((st = stage_batch(sv, k, src, dst, w, true))) return st;
   const size_t K = (size_t)sv->kcap;
   return run_mode(sv, mode, k, sv->ubuf, sv->ubuf + K, sv->ubuf + 2 * K, flow, true);
 }
@@ -635,7 +692,7 @@ int scheduled_updates(dmf_solver *sv, dmf_sched *sched, int action, int32_t k, c
   if (st) return st;
   if (!sv->solved) return fail(DMF_ERR_NOT_SOLVED, "apply_updates before a solve");
   if (action >= DMF_SCHED_ACTIONS) return fail(DMF_ERR_INVALID_ARG, "unknown action %d", action);
-  if ((st = stage_batch(sv, k, src, dst, w))) return st;
+  if ((st = stage_batch(sv, k, src, dst, w, false))) return st;
   dmf_solver::SchedRecord rec{};
   int picked = 0;
   if ((st = batch_features(sv, action < 0 ? sched : nullptr, k, rec.feat, &picked))) return st;
@@ -643,6 +700,7 @@ int scheduled_updates(dmf_solver *sv, dmf_sched *sched, int action, int32_t k, c
   int64_t f = 0;
   if ((st = apply_action(sv, picked, k, &f))) return st;
   rec.action = picked;
+  resolve_ms(sv);
   rec.ms = (float)sv->st.last_ms;
   rec.flow = f;
   if (sv->records.size() < (1u << 20)) sv->records.push_back(rec);
@@ -658,6 +716,7 @@ int device_updates(dmf_solver *sv, int mode, int32_t k, const int32_t *src, cons
   if (mode == MODE_DYNAMIC && !sv->solved) return fail(DMF_ERR_NOT_SOLVED, "apply_updates before a solve");
   CK(cudaSetDevice(sv->dev), "cudaSetDevice");
   if ((st = ensure_ubuf(sv, k))) return st;  // for the per-update arc scratch
+  sv->direct = false;
   return run_mode(sv, mode, k, src, dst, w, flow, false);
 }
 
@@ -778,6 +837,7 @@ int dmf_static_maxflow_noalloc(int32_t n, int32_t m, const int32_t *d_index, con
     p.res = d_res;
     p.uarc = nullptr;
     p.uold = nullptr;
+    p.hres = nullptr;
     p.ctrl = ctrl;
     p.mode = MODE_STATIC;
     p.variant = DMF_VARIANT_DATA;
@@ -950,12 +1010,19 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->inl, 0, N, S);
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->lst, 0, 4, S);
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->excess, 0, 8 * N, S);
-  if (e == cudaSuccess) e = cudaMallocHost(&sv->h_ctrl, sizeof(Ctrl));
+  if (e == cudaSuccess) e = cudaHostAlloc((void **)&sv->h_res, sizeof(HostResult), cudaHostAllocMapped);
+  if (e == cudaSuccess) std::memset((void *)sv->h_res, 0, sizeof(HostResult));
+  if (e == cudaSuccess) e = cudaMemsetAsync(sv->ctrl, 0, sizeof(Ctrl), S);
   if (e == cudaSuccess) e = cudaEventCreate(&sv->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&sv->ev1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(S);
   if (e != cudaSuccess) return cuda_fail(e, "solver upload");
-  if ((st = ensure_ubuf(sv, 1024))) return st;
+  // staging for an eighth of the arcs up front, up to 2^18 updates, and for 3%
+  // beyond that on the device (a call that has to grow it waits for the device
+  // and for the allocations: ms, at times tens of ms)
+  const size_t some = std::min<size_t>(M / 8, 1 << 18);
+  if ((st = ensure_ubuf(sv, (int)std::max<size_t>({1024, some, M / 32})))) return st;
+  if ((st = ensure_host_ubuf(sv, (int)std::max<size_t>(1024, some)))) return st;
   // sources (and, for batched instances, roles, instance ids, per-instance flows)
   {
     const std::vector<int> one(1, s);
@@ -982,7 +1049,8 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
         return cuda_fail(cudaGetLastError(), "pinned mask");
       if (cudaMemcpy(sv->role, ms->role.data(), ms->role.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
           cudaMemcpy(sv->inst, ms->inst.data(), 4 * ms->inst.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-          cudaMallocHost(&sv->h_inst_flow, 8 * (size_t)ms->count) != cudaSuccess)
+          cudaHostAlloc((void **)&sv->h_inst_flow, 8 * (size_t)ms->count, cudaHostAllocMapped) != cudaSuccess ||
+          cudaMemset(sv->inst_flow, 0, 8 * (size_t)ms->count) != cudaSuccess)
         return cuda_fail(cudaGetLastError(), "batched-instance upload");
     }
   }
@@ -1154,13 +1222,14 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
       S = sv->own_stream;
     }
     const int cnt = sv->ninst;
-    Ctrl *h_ctrl = nullptr;
+    HostResult *h_res = nullptr;
     long long *h_fl = nullptr;
-    CK(cudaMallocHost(&h_ctrl, sizeof(Ctrl) * (size_t)steps), "pinned control");
-    if (cudaMallocHost(&h_fl, 8 * (size_t)steps * cnt) != cudaSuccess) {
-      cudaFreeHost(h_ctrl);
+    CK(cudaHostAlloc((void **)&h_res, sizeof(HostResult) * (size_t)steps, cudaHostAllocMapped), "pinned results");
+    if (cudaHostAlloc((void **)&h_fl, 8 * (size_t)steps * cnt, cudaHostAllocMapped) != cudaSuccess) {
+      cudaFreeHost(h_res);
       return fail(DMF_ERR_OOM, "pinned flows");
     }
+    sv->direct = false;
     // step b uses its own range of round ids, relabel epochs and batch stamp
     constexpr unsigned kRoundStride = 1u << 20, kRelabelStride = 1u << 18;
     KernelFn fn = pick_kernel(sv->tile, sv->minb);
@@ -1172,9 +1241,8 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
         p.relabel_base = sv->relabel_base + (unsigned)b * kRelabelStride;
         p.trace = nullptr;
         p.probe = 0;
-        cudaError_t e = cudaMemsetAsync(sv->ctrl, 0, sizeof(Ctrl), S);
-        if (e == cudaSuccess && sv->inst_flow) e = cudaMemsetAsync(sv->inst_flow, 0, 8 * (size_t)cnt, S);
-        if (e != cudaSuccess) return e;
+        p.hres = h_res + b;
+        p.hflow = h_fl + (size_t)b * cnt;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sv->grid);
         cfg.blockDim = dim3(sv->block);
@@ -1185,15 +1253,7 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, fn, p);
-        if (e != cudaSuccess) return e;
-        e = cudaMemcpyAsync(h_ctrl + b, sv->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, S);
-        if (e == cudaSuccess) {
-          if (sv->inst_flow)
-            e = cudaMemcpyAsync(h_fl + (size_t)b * cnt, sv->inst_flow, 8 * (size_t)cnt, cudaMemcpyDeviceToHost, S);
-          else
-            e = cudaMemcpyAsync(h_fl + b, &sv->ctrl->flow, 8, cudaMemcpyDeviceToHost, S);
-        }
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, p);
         if (e != cudaSuccess) return e;
       }
       return cudaSuccess;
@@ -1217,7 +1277,7 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
-      cudaFreeHost(h_ctrl);
+      cudaFreeHost(h_res);
       cudaFreeHost(h_fl);
       return cuda_fail(e, use_graph ? "graph-captured batch loop" : "batch loop");
     }
@@ -1227,7 +1287,7 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
     int rc = DMF_OK;
     unsigned outer = 0;
     for (int b = 0; b < steps && !rc; b++) {
-      const Ctrl &c = h_ctrl[b];
+      const Ctrl &c = h_res[b].c;
       outer += (unsigned)c.st_outer;
       if (c.err) rc = fail(c.err & ERR_TIMEOUT ? DMF_ERR_TIMEOUT
                            : c.err & ERR_NO_CONV ? DMF_ERR_NO_CONVERGENCE
@@ -1235,6 +1295,8 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
                                                                                       : DMF_ERR_CUDA,
                            "step %d: device error flags 0x%x (update %d)", b, c.err, c.err_info);
     }
+    if (!sv->inst_flow)  // a single-instance solver: its flow is in the control block
+      for (int b = 0; b < steps; b++) h_fl[b] = h_res[b].c.flow;
     for (size_t i = 0; i < (size_t)steps * cnt; i++) flows[i] = h_fl[i];
     sv->round_base += (unsigned)steps * kRoundStride;
     sv->relabel_base += (unsigned)steps * kRelabelStride;
@@ -1244,12 +1306,13 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
       for (int64_t f : sv->flows) tot += f;
       sv->st.flow = tot;
       sv->st.last_ms = t_ms;
+      sv->ms_pending = false;
       sv->st.outer_iters = outer;
       sv->side_valid = false;
     } else {
       sv->solved = false;
     }
-    cudaFreeHost(h_ctrl);
+    cudaFreeHost(h_res);
     cudaFreeHost(h_fl);
     return rc ? rc : ok();
   });
@@ -1268,6 +1331,7 @@ int dmf_autotune(dmf_solver *sv, int32_t repeats, dmf_opts *chosen) {
       for (int r = 0; r < repeats; r++) {
         st = host_updates(sv, MODE_RECOMPUTE, 0, nullptr, nullptr, nullptr, nullptr);
         if (st) return st;
+        resolve_ms(sv);
         b = std::min(b, sv->st.last_ms);
       }
       *out = b;
@@ -1368,10 +1432,12 @@ int dmf_get_cut(dmf_solver *sv, uint8_t *sink_side) {
     CK(cudaSetDevice(sv->dev), "cudaSetDevice");
     if (!sv->side_valid) {
       int64_t f = sv->st.flow;
+      resolve_ms(sv);
       dmf_stats keep = sv->st;
       int st = run_mode(sv, MODE_CUT, 0, nullptr, nullptr, nullptr, nullptr, false);
       if (st) return st;
       sv->st = keep;
+      sv->ms_pending = false;
       sv->st.flow = f;
       sv->side_valid = true;
     }
@@ -1412,7 +1478,7 @@ int dmf_trace_items(dmf_solver *sv, int32_t cap, int64_t *items, int64_t *hubs, 
                     int64_t *slow_v) {
   return guarded([&]() -> int {
     if (!sv || cap < 0 || (cap > 0 && (!items || !hubs))) return fail(DMF_ERR_INVALID_ARG, "bad arguments");
-    const int len = std::min(std::min(sv->h_ctrl ? sv->h_ctrl->trace_len : 0, sv->trace_cap), cap);
+    const int len = std::min(std::min(sv->h_res ? sv->h_res->c.trace_len : 0, sv->trace_cap), cap);
     if (len <= 0) return ok();
     std::vector<unsigned long long> h(4 * (size_t)len);
     CK(cudaSetDevice(sv->dev), "cudaSetDevice");
@@ -1431,7 +1497,7 @@ int dmf_trace_items(dmf_solver *sv, int32_t cap, int64_t *items, int64_t *hubs, 
 int dmf_trace_blocks(dmf_solver *sv, int32_t cap, int64_t *block_ns) {
   return guarded([&]() -> int {
     if (!sv || cap < 0 || (cap > 0 && !block_ns)) return fail(DMF_ERR_INVALID_ARG, "bad arguments");
-    const int len = std::min(std::min(sv->h_ctrl ? sv->h_ctrl->trace_len : 0, sv->trace_cap), cap);
+    const int len = std::min(std::min(sv->h_res ? sv->h_res->c.trace_len : 0, sv->trace_cap), cap);
     if (len <= 0) return ok();
     std::vector<unsigned long long> h(4 * (size_t)len);
     CK(cudaSetDevice(sv->dev), "cudaSetDevice");
@@ -1445,7 +1511,7 @@ int dmf_trace_blocks(dmf_solver *sv, int32_t cap, int64_t *block_ns) {
 int dmf_trace_get(dmf_solver *sv, int32_t cap, int32_t *kinds, double *t_us, int32_t *count) {
   return guarded([&]() -> int {
     if (!sv || !count || cap < 0 || (cap > 0 && (!kinds || !t_us))) return fail(DMF_ERR_INVALID_ARG, "bad arguments");
-    const int len = std::min(sv->h_ctrl ? sv->h_ctrl->trace_len : 0, sv->trace_cap);
+    const int len = std::min(sv->h_res ? sv->h_res->c.trace_len : 0, sv->trace_cap);
     *count = len;
     if (len == 0 || cap == 0) return ok();
     std::vector<unsigned long long> h(4 * (size_t)len);
@@ -1462,6 +1528,7 @@ int dmf_trace_get(dmf_solver *sv, int32_t cap, int32_t *kinds, double *t_us, int
 
 int dmf_stats_get(const dmf_solver *sv, dmf_stats *st) {
   if (!sv || !st) return fail(DMF_ERR_INVALID_ARG, "null argument");
+  resolve_ms(sv);
   *st = sv->st;
   return ok();
 }
@@ -1472,7 +1539,7 @@ int dmf_solver_features(dmf_solver *sv, int32_t k, const int32_t *src, const int
     int st = check_updates_args(sv, k, src, dst, w);
     if (st) return st;
     if (!feat) return fail(DMF_ERR_INVALID_ARG, "null feature output");
-    if ((st = stage_batch(sv, k, src, dst, w))) return st;
+    if ((st = stage_batch(sv, k, src, dst, w, false))) return st;
     int action = 0;
     if ((st = batch_features(sv, nullptr, k, feat, &action))) return st;
     return ok();
@@ -1542,7 +1609,9 @@ int dmf_solver_copy_state(dmf_solver *dst, const dmf_solver *src) {
     dst->epoch = std::max(dst->epoch, src->epoch);
     dst->solved = src->solved;
     dst->side_valid = src->side_valid;
+    resolve_ms(src);
     dst->st = src->st;
+    dst->ms_pending = false;
     dst->flows = src->flows;
     return ok();
   });
