@@ -138,7 +138,8 @@ __device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh,
       const int h = __ldcg(p.height + v);
       scan[j] = first ? h : sh.scan[j * kBlock + (int)threadIdx.x];
       if (h != p.n && inst_on(p, v)) {        // neither a source nor dead
-        if (first && h == L0) scan[j] = UNV;  // the frontier
+        // the frontier, and what a warp that began earlier has labelled already
+        if (first && h >= L0) scan[j] = UNV;
         beg[j] = __ldg(p.off + v);
         const int deg = __ldg(p.off + v + 1) - beg[j];
         mask[j] = (unsigned)min(deg, 255) << 8;
