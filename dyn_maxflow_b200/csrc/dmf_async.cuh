@@ -121,6 +121,94 @@ __device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool
 // Labels only fall and every fall is seen by its owner, so once no vertex has a
 // label below the one it last relaxed from (ph_async_settled, between two
 // barriers) the labels are the exact distances.
+// Relaxes the tails of a long row's residual in-arcs, by a whole warp.
+__device__ __forceinline__ void async_relax_row(const Params &p, int v, int h, LStats &ls) {
+  const int b = __ldg(p.off + v), e = __ldg(p.off + v + 1);
+  for (int a = b + (int)(threadIdx.x & 31); a < e; a += 32) {
+    const int w = __ldg(p.adj + a);
+    ls.barcs++;
+    const int cur = __ldcg(p.height + w);
+    if (cur > h + 1 && cur != p.n && __ldcg(p.res + __ldg(p.par + a)) > 0) atomicMin(p.height + w, h + 1);
+  }
+  __syncwarp();
+}
+
+// One window per warp: the heads that can be labelled over the vertex's arcs sit
+// in registers, so a hop is a poll, a vote and the atomics.
+__device__ __forceinline__ void async_bfs_one(const Params &p, AsyncShared &sh, const AsyncOwn &own, int L0, bool first,
+                                              LStats &ls) {
+  Ctrl *c = p.ctrl;
+  const int lane = threadIdx.x & 31, v = own.first + lane;
+  const bool mine = own.count > 0 && v < p.n;
+  int scan = INT_MIN, beg = 0, deg = 0, nh = 0;
+  int hd[kSmallMax];
+#pragma unroll
+  for (int k = 0; k < kSmallMax; k++) hd[k] = 0;
+  if (mine) {
+    const int h = __ldcg(p.height + v);
+    scan = first ? h : sh.scan[threadIdx.x];
+    if (h != p.n && inst_on(p, v)) {  // neither a source nor dead
+      // the frontier, and what a warp that began earlier has labelled already
+      if (first && h >= L0) scan = UNV;
+      beg = __ldg(p.off + v);
+      deg = __ldg(p.off + v + 1) - beg;
+      if (deg <= kSmallMax) {
+        int w[kSmallMax];
+        bool ok[kSmallMax];
+#pragma unroll
+        for (int k = 0; k < kSmallMax; k++) {
+          ok[k] = false;
+          w[k] = 0;
+          if (k >= deg) continue;
+          w[k] = __ldg(p.adj + beg + k);
+          ok[k] = __ldcg(p.res + __ldg(p.par + beg + k)) > 0 && __ldcg(p.height + w[k]) != p.n;
+        }
+#pragma unroll
+        for (int k = 0; k < kSmallMax; k++) {
+          if (!ok[k]) continue;
+#pragma unroll
+          for (int j = 0; j < kSmallMax; j++)
+            if (j == nh) hd[j] = w[k];
+          nh++;
+        }
+      }
+    }
+  }
+  const bool wide = deg > kSmallMax;
+  const bool any_wide = __any_sync(0xffffffffu, wide), many = __any_sync(0xffffffffu, nh > 4);
+  AsyncIdle st;
+  for (int poll = 0;; poll++) {
+    const int h = mine ? ld_rlx(p.height + v) : INT_MAX;
+    const bool need = h < scan;
+    if (!__any_sync(0xffffffffu, need)) {
+      if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[0], &c->astop, &c->err)) break;
+      continue;
+    }
+    if (need) {
+      scan = h;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (k < nh) atomicMin(p.height + hd[k], h + 1);
+      if (many) {
+#pragma unroll
+        for (int k = 4; k < kSmallMax; k++)
+          if (k < nh) atomicMin(p.height + hd[k], h + 1);
+      }
+      ls.barcs += (unsigned)nh;
+    }
+    if (any_wide) {
+      unsigned todo = __ballot_sync(0xffffffffu, need && wide);
+      while (todo) {  // longer rows by the whole warp
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        async_relax_row(p, own.first + src, __shfl_sync(0xffffffffu, h, src), ls);
+      }
+    }
+    if (async_busy(sh, st, &c->aidle[0])) break;
+  }
+  sh.scan[threadIdx.x] = scan;
+}
+
 template <int W>
 __device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh, const AsyncOwn &own, int L0, bool first,
                                                LStats &ls) {
@@ -185,16 +273,7 @@ __device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh,
       while (wide) {  // longer rows by the whole warp
         const int src = __ffs(wide) - 1;
         wide &= wide - 1;
-        const int v = own.first + j * own.step + src;
-        const int b = __shfl_sync(0xffffffffu, beg[j], src), e = __ldg(p.off + v + 1);
-        const int hv = __shfl_sync(0xffffffffu, h[j], src);
-        for (int a = b + lane; a < e; a += 32) {
-          const int w = __ldg(p.adj + a);
-          ls.barcs++;
-          const int cur = __ldcg(p.height + w);
-          if (cur > hv + 1 && cur != p.n && __ldcg(p.res + __ldg(p.par + a)) > 0) atomicMin(p.height + w, hv + 1);
-        }
-        __syncwarp();
+        async_relax_row(p, own.first + j * own.step + src, __shfl_sync(0xffffffffu, h[j], src), ls);
       }
     }
     if (async_busy(sh, st, &c->aidle[0])) break;
@@ -214,8 +293,25 @@ __device__ __forceinline__ void ph_async_bfs(const Params &p, AsyncShared &sh, i
     c->adepth = 0;
   }
   async_begin(sh);
-  if (own.count <= 1) async_bfs_loop<1>(p, sh, own, L0, first, ls);
+  if (own.count <= 1) async_bfs_one(p, sh, own, L0, first, ls);
   else async_bfs_loop<kAsyncWin>(p, sh, own, L0, first, ls);
+}
+
+// The seeds of a relabel of a deep solve: labels only (the frontier and active
+// lists of ph_bfs_init are not used there; 3.5 us instead of 17 at 65,536
+// vertices).
+__device__ __forceinline__ void ph_deep_init(const Params &p) {
+  const int nt = gridDim.x * blockDim.x;
+  int pos = 0;
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < p.n; v += nt) {
+    const bool is_dead = __ldcg(p.dead + v) != 0;
+    const long long ex = __ldcg(p.excess + v);
+    if (is_dead || !inst_on(p, v)) continue;
+    const bool src = is_src(p, v), snk = is_snk(p, v);
+    p.height[v] = src ? p.n : (snk || ex < 0) ? 0 : UNV;
+    if (!src && !snk && ex > 0) pos++;
+  }
+  block_add_int(0, &p.ctrl->pos_count, pos);
 }
 
 // After a barrier: counts the vertices whose label fell since they last relaxed
@@ -262,6 +358,97 @@ __device__ __forceinline__ void ph_async_finalize(const Params &p, bool write_si
 // races are those of the rounds.  Ends when no vertex is active, or after
 // budget_ns (set by the grid's first thread): the next relabel then gives exact
 // distances again.
+// One window per warp, every narrow vertex of it with at most D arcs: heads,
+// partners and the label (only the owner changes it) sit in registers, and a
+// discharge is one round of loads, up to `cycles` pushes and relabels on what
+// they gave, and the atomics.
+template <int D>
+__device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh, const AsyncOwn &own, bool live, bool lead,
+                                               unsigned long long t0, unsigned long long budget_ns, LStats &ls) {
+  Ctrl *c = p.ctrl;
+  const int lane = threadIdx.x & 31, v = own.first + lane;
+  int beg = 0, deg = 0, h = p.n;
+  int hd[D], pa[D];
+  if (live) {
+    beg = __ldg(p.off + v);
+    deg = __ldg(p.off + v + 1) - beg;
+    h = __ldcg(p.height + v);
+  }
+  const bool wide = deg > kSmallMax;
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    hd[k] = !wide && k < deg ? __ldg(p.adj + beg + k) : 0;
+    pa[k] = !wide && k < deg ? __ldg(p.par + beg + k) : 0;
+  }
+  const bool any_wide = __any_sync(0xffffffffu, wide);
+  TileGroup<32> wg;
+  AsyncIdle st;
+  for (int poll = 0;; poll++) {
+    const long long ex = live ? ld_rlx(p.excess + v) : 0;
+    const bool act = ex > 0 && h < p.n;
+    if (lead && (poll & 7) == 0 && globaltimer() - t0 > budget_ns) atomicExch(&c->astop, 1);
+    if (!__any_sync(0xffffffffu, act)) {
+      if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) break;
+      continue;
+    }
+    if (act && !wide) {
+      int rr[D], hw[D], dd[D];
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        rr[k] = k < deg ? __ldcg(p.res + beg + k) : 0;
+        hw[k] = k < deg ? __ldcg(p.height + hd[k]) : INT_MAX;
+        dd[k] = 0;
+      }
+      ls.visits++;
+      ls.arcs += (unsigned)deg;
+      long long left = ex;
+      const int h0 = h;
+      for (int cyc = 0; cyc < p.cycles && left > 0 && h < p.n; cyc++) {
+#pragma unroll
+        for (int k = 0; k < D; k++) {
+          if (rr[k] > 0 && hw[k] < h) {
+            const int d = (int)(rr[k] < left ? rr[k] : left);
+            dd[k] += d;
+            rr[k] -= d;
+            left -= d;
+          }
+        }
+        if (left > 0) {  // every admissible arc is saturated: relabel
+          int mh = INT_MAX;
+#pragma unroll
+          for (int k = 0; k < D; k++)
+            if (rr[k] > 0) mh = min(mh, hw[k]);
+          h = mh >= p.n ? p.n : mh + 1;
+          ls.relabels++;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        if (dd[k] > 0) {
+          atomicSub(p.res + beg + k, dd[k]);
+          push_excess(p, hd[k], dd[k], ls);
+          atomicAdd(p.res + pa[k], dd[k]);
+          ls.pushes++;
+        }
+      }
+      if (h != h0) *(volatile int *)(p.height + v) = h;
+      if (left != ex) atomic_add_ll(p.excess + v, left - ex);
+    }
+    if (any_wide) {
+      unsigned todo = __ballot_sync(0xffffffffu, act && wide);
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        discharge(wg, p, own.first + src, 0, 0, false, ls, nullptr);
+        __syncwarp();
+        if (lane == src) h = __ldcg(p.height + v);
+      }
+    }
+    if (threadIdx.x == 0 && (poll & 7) == 0 && ld_rlx(&c->astop)) *(volatile int *)&sh.stop = 1;
+    if (async_busy(sh, st, &c->aidle[1])) break;
+  }
+}
+
 __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, unsigned long long budget_ns,
                                               LStats &ls) {
   Ctrl *c = p.ctrl;
@@ -281,23 +468,28 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
     const int v = own.first + j * own.step + lane;
     if (v < p.n && !__ldcg(p.dead + v) && !is_term(p, v) && inst_on(p, v)) live |= 1u << j;
   }
+  if (own.count <= 1) {
+    const int v = own.first + lane;
+    const int deg = live & 1 ? deg_of(p, v) : 0;
+    if (__any_sync(0xffffffffu, deg > 4 && deg <= kSmallMax))
+      async_push_one<kSmallMax>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
+    else
+      async_push_one<4>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
+    __syncwarp();
+    sink_flush(p, ls);
+    return;
+  }
   TileGroup<32> wg;
   AsyncIdle st;
   for (int poll = 0;; poll++) {
     unsigned have = 0;  // windows in which this lane's vertex holds excess
-    long long ex0 = 0;
-    if (own.count <= 1) {
-      if (live & 1) ex0 = ld_rlx(p.excess + own.first + lane);
-      have = ex0 > 0;
-    } else {
-      long long ex[kAsyncWin];
+    long long ex[kAsyncWin];
 #pragma unroll
-      for (int j = 0; j < kAsyncWin; j++)
-        ex[j] = (live >> j) & 1 ? ld_rlx(p.excess + own.first + j * own.step + lane) : 0;
+    for (int j = 0; j < kAsyncWin; j++)
+      ex[j] = (live >> j) & 1 ? ld_rlx(p.excess + own.first + j * own.step + lane) : 0;
 #pragma unroll
-      for (int j = 0; j < kAsyncWin; j++)
-        if (ex[j] > 0) have |= 1u << j;
-    }
+    for (int j = 0; j < kAsyncWin; j++)
+      if (ex[j] > 0) have |= 1u << j;
     bool any = false;
     if (__any_sync(0xffffffffu, have)) {
 #pragma unroll 1
@@ -307,7 +499,7 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
         long long x = 0;
         int h = p.n, beg = 0, deg = 0;
         if ((have >> j) & 1) {
-          x = own.count <= 1 ? ex0 : __ldcg(p.excess + v);
+          x = __ldcg(p.excess + v);
           h = __ldcg(p.height + v);
           beg = __ldg(p.off + v);
           deg = __ldg(p.off + v + 1) - beg;

@@ -2362,7 +2362,8 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     }
     kind = TR_BFS_INIT;
     items = hubitems = 0;
-    ph_bfs_init(p, slot_out(), it == 0 && revive, it == 0 && !revive, listed);
+    if (deep) ph_deep_init(p);
+    else ph_bfs_init(p, slot_out(), it == 0 && revive, it == 0 && !revive, listed);
     if (!next()) return;
     if (lead) c->st_outer++;
     const int P = sc->pos_count;
