@@ -87,14 +87,30 @@ __device__ __forceinline__ void async_begin(AsyncShared &sh) {
   __syncthreads();
 }
 
-// A warp that found work in its last poll.
-__device__ __forceinline__ bool async_busy(AsyncShared &sh, AsyncIdle &st, int *idle_blocks) {
+// The block's look at the phase's stop word, every 8th poll whatever the polls
+// find: a warp that finds work at every other poll (excess that goes to and fro
+// between two windows until its labels reach n) would else never look.
+__device__ __forceinline__ void async_look(AsyncShared &sh, int poll, const int *stop, const int *err) {
+  if (threadIdx.x == 0 && (poll & 7) == 7 && (ld_rlx(stop) || ld_rlx(err) || poll >= kMaxPolls))
+    *(volatile int *)&sh.stop = 1;
+}
+
+// A warp that found work; called before it does it, so that a long piece of work
+// does not look like quiet.
+__device__ __forceinline__ void async_wake(AsyncShared &sh, AsyncIdle &st, int *idle_blocks) {
   st.quiet = 0;
   if (st.idle) {
     st.idle = false;
     if ((threadIdx.x & 31) == 0 && atomicSub(&sh.idle_warps, 1) == (int)(blockDim.x >> 5)) atomicSub(idle_blocks, 1);
   }
-  return *(volatile int *)&sh.stop != 0;
+}
+__device__ __forceinline__ bool async_stopped(const AsyncShared &sh) { return *(const volatile int *)&sh.stop != 0; }
+
+// Every warp has left: a block that stopped while one of its warps had just woken
+// is counted as idle again, or the others would wait for it.
+__device__ __forceinline__ void async_end(AsyncShared &sh, int *idle_blocks) {
+  __syncthreads();
+  if (threadIdx.x == 0 && sh.idle_warps < (int)(blockDim.x >> 5)) atomicAdd(idle_blocks, 1);
 }
 
 // A warp whose last poll found nothing; true: leave the phase.  The block's
@@ -112,7 +128,7 @@ __device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool
       (ld_rlx(idle_blocks) >= (int)gridDim.x || ld_rlx(stop) || ld_rlx(err) || poll >= kMaxPolls))
     *(volatile int *)&sh.stop = 1;
   if (!owner) __nanosleep(200);
-  return *(volatile int *)&sh.stop != 0;
+  return async_stopped(sh);
 }
 
 // Global relabel from the labels a level-synchronous BFS left after its level
@@ -184,6 +200,7 @@ __device__ __forceinline__ void async_bfs_one(const Params &p, AsyncShared &sh, 
       if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[0], &c->astop, &c->err)) break;
       continue;
     }
+    async_wake(sh, st, &c->aidle[0]);
     if (need) {
       scan = h;
 #pragma unroll
@@ -204,7 +221,7 @@ __device__ __forceinline__ void async_bfs_one(const Params &p, AsyncShared &sh, 
         async_relax_row(p, own.first + src, __shfl_sync(0xffffffffu, h, src), ls);
       }
     }
-    if (async_busy(sh, st, &c->aidle[0])) break;
+    if (async_stopped(sh)) break;
   }
   sh.scan[threadIdx.x] = scan;
 }
@@ -256,6 +273,7 @@ __device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh,
       if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[0], &c->astop, &c->err)) break;
       continue;
     }
+    async_wake(sh, st, &c->aidle[0]);
 #pragma unroll
     for (int j = 0; j < W; j++) {
       const bool need = h[j] < scan[j];
@@ -276,7 +294,7 @@ __device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh,
         async_relax_row(p, own.first + j * own.step + src, __shfl_sync(0xffffffffu, h[j], src), ls);
       }
     }
-    if (async_busy(sh, st, &c->aidle[0])) break;
+    if (async_stopped(sh)) break;
   }
 #pragma unroll
   for (int j = 0; j < W; j++) sh.scan[j * kBlock + (int)threadIdx.x] = scan[j];
@@ -295,6 +313,7 @@ __device__ __forceinline__ void ph_async_bfs(const Params &p, AsyncShared &sh, i
   async_begin(sh);
   if (own.count <= 1) async_bfs_one(p, sh, own, L0, first, ls);
   else async_bfs_loop<kAsyncWin>(p, sh, own, L0, first, ls);
+  async_end(sh, &c->aidle[0]);
 }
 
 // The seeds of a relabel of a deep solve: labels only (the frontier and active
@@ -387,10 +406,12 @@ __device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh,
     const long long ex = live ? ld_rlx(p.excess + v) : 0;
     const bool act = ex > 0 && h < p.n;
     if (lead && (poll & 7) == 0 && globaltimer() - t0 > budget_ns) atomicExch(&c->astop, 1);
+    async_look(sh, poll, &c->astop, &c->err);
     if (!__any_sync(0xffffffffu, act)) {
       if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) break;
       continue;
     }
+    async_wake(sh, st, &c->aidle[1]);
     if (act && !wide) {
       int rr[D], hw[D], dd[D];
 #pragma unroll
@@ -444,8 +465,7 @@ __device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh,
         if (lane == src) h = __ldcg(p.height + v);
       }
     }
-    if (threadIdx.x == 0 && (poll & 7) == 0 && ld_rlx(&c->astop)) *(volatile int *)&sh.stop = 1;
-    if (async_busy(sh, st, &c->aidle[1])) break;
+    if (async_stopped(sh)) break;
   }
 }
 
@@ -475,7 +495,7 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
       async_push_one<kSmallMax>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
     else
       async_push_one<4>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
-    __syncwarp();
+    async_end(sh, &c->aidle[1]);
     sink_flush(p, ls);
     return;
   }
@@ -505,6 +525,7 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
           deg = __ldg(p.off + v + 1) - beg;
         }
         const bool act = x > 0 && h < p.n;
+        if (__any_sync(0xffffffffu, act)) async_wake(sh, st, &c->aidle[1]);
         any |= act;
         if (act && deg <= kSmallMax) {
           ls.visits++;
@@ -521,12 +542,13 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
       any = __any_sync(0xffffffffu, any);
     }
     if (lead && (poll & 7) == 0 && globaltimer() - t0 > budget_ns) atomicExch(&c->astop, 1);
+    async_look(sh, poll, &c->astop, &c->err);
     if (any) {
-      if (threadIdx.x == 0 && (poll & 7) == 0 && ld_rlx(&c->astop)) *(volatile int *)&sh.stop = 1;
-      if (async_busy(sh, st, &c->aidle[1])) break;
+      if (async_stopped(sh)) break;
     } else if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) {
       break;
     }
   }
+  async_end(sh, &c->aidle[1]);
   sink_flush(p, ls);
 }
