@@ -18,6 +18,8 @@
 // there a level is real work and the worklists save polling every vertex.  A
 // graph that needs 24 levels will need hundreds of short phases.
 constexpr int kDeepLevels = 24;
+// Levels after which the partial revival of a batch gives up on such a graph.
+constexpr int kReviveLevels = 8;
 // Windows of 32 vertices per warp at most: bounds the vertices a graph may
 // have (kAsyncWin * 32 * resident warps) and the per-vertex shared memory.
 constexpr int kAsyncWin = 4;
@@ -460,7 +462,7 @@ __device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh,
       while (todo) {
         const int src = __ffs(todo) - 1;
         todo &= todo - 1;
-        discharge(wg, p, own.first + src, 0, 0, false, ls, nullptr);
+        discharge(wg, p, own.first + src, 0, false, ls, nullptr);
         __syncwarp();
         if (lane == src) h = __ldcg(p.height + v);
       }
@@ -529,13 +531,13 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
         any |= act;
         if (act && deg <= kSmallMax) {
           ls.visits++;
-          discharge_small(p, v, beg, deg, x, h, 0, 0, false, ls);
+          discharge_small(p, v, beg, deg, x, h, 0, false, ls);
         }
         unsigned wide = __ballot_sync(0xffffffffu, act && deg > kSmallMax);
         while (wide) {
           const int src = __ffs(wide) - 1;
           wide &= wide - 1;
-          discharge(wg, p, __shfl_sync(0xffffffffu, v, src), 0, 0, false, ls, nullptr);
+          discharge(wg, p, __shfl_sync(0xffffffffu, v, src), 0, false, ls, nullptr);
           __syncwarp();
         }
       }

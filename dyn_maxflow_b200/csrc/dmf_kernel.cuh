@@ -933,7 +933,9 @@ __device__ __forceinline__ bool bu_batch(const Params &p, int first, int end, in
 #pragma unroll
   for (int k = 0; k < kBatch; k++) {
     const int a = first + k * stride;
-    r[k] = a < end ? __ldcg(p.res + a) : 0;
+    // through L1: residuals do not change during a relabel, and the rows of a
+    // warp's vertices share sectors
+    r[k] = a < end ? p.res[a] : 0;
     w[k] = a < end ? __ldg(p.adj + a) : -1;
   }
   bool hit = false;
@@ -1337,8 +1339,15 @@ __device__ __forceinline__ void ph_dead_revive(const Params &p, const Slot *in, 
 // appends to buffers r&1 with tails wtail/whtail[r%3]; tails are triple-buffered
 // for the same reason as the phase slots.
 
-__device__ __forceinline__ void enqueue(const Params &p, int r, unsigned round_id, int v) {
-  if (atomicExch(p.stamp + v, (int)round_id) == (int)round_id) return;
+// A vertex joins the next round's list once, without a mark of its own.  Every
+// vertex with excess is in the round's list.  Its discharge takes what it moved
+// out of the excess with one atomic at its end and queues the vertex when that
+// leaves something (leftover, or what arrived meanwhile); a push queues its head
+// when it raised the excess from zero or below to above.  The excess word orders
+// these: within a round it falls once at most, so only one of them sees the
+// change.  (A stamp exchanged by every push put a second returning atomic, on
+// the busiest hubs' words, behind the first: R-MAT 20 push round 83 -> 58 us.)
+__device__ __forceinline__ void enqueue(const Params &p, int r, int v) {
   if (deg_of(p, v) > p.hub_deg) append_hub(p, p.wh[r & 1], &p.ctrl->whtail[r % 3], v);
   else append(p.wq[r & 1], &p.ctrl->wtail[r % 3], v);
 }
@@ -1363,31 +1372,23 @@ __device__ __forceinline__ void sink_flush(const Params &p, LStats &ls) {
   ls.to_sink = 0;
 }
 
-__device__ __forceinline__ void push_arc(const Params &p, int a, int w, int d, int r, unsigned round_id, bool enq,
-                                         LStats &ls) {
+__device__ __forceinline__ void push_arc(const Params &p, int a, int w, int d, int r, bool enq, LStats &ls) {
   atomicSub(p.res + a, d);
   atomicAdd(p.res + __ldg(p.par + a), d);
   long long old = push_excess(p, w, d, ls);
   ls.pushes++;
-  if (enq && !is_term(p, w) && old + d > 0) enqueue(p, r, round_id, w);
+  if (enq && old <= 0 && old + d > 0 && !is_term(p, w)) enqueue(p, r, w);
 }
 
 // Arcs a lane handles together in a tile discharge.
 constexpr int kPushBatch = 4;
 
 
-// Queues the heads x[k] marked in `cand` for round r+1 (each at most once per
-// round, by its stamp): all stamp exchanges in flight together, then all degree
-// reads, then one reservation for the non-hub heads (hubs go to the chunk queue).
+// Queues the vertices x[k] marked in `keep` for round r+1: all degree reads in
+// flight together, then one reservation for the non-hub ones (hubs go to the
+// chunk queue).
 template <int K>
-__device__ __forceinline__ void enqueue_batch(const Params &p, const int (&x)[K], unsigned cand, int r,
-                                              unsigned round_id) {
-  unsigned keep = 0;
-#pragma unroll
-  for (int k = 0; k < K; k++)
-    if ((cand >> k) & 1)
-      if (atomicExch(p.stamp + x[k], (int)round_id) != (int)round_id) keep |= 1u << k;
-  if (!keep) return;
+__device__ __forceinline__ void enqueue_batch(const Params &p, const int (&x)[K], unsigned keep, int r) {
   int dg[K];
 #pragma unroll
   for (int k = 0; k < K; k++) dg[k] = ((keep >> k) & 1) ? deg_of(p, x[k]) : 0;
@@ -1416,7 +1417,7 @@ __device__ __forceinline__ void enqueue_batch(const Params &p, const int (&x)[K]
 // partner residuals; heads whose excess became positive are queued (enq).
 template <int K>
 __device__ __forceinline__ void push_batch(const Params &p, const int (&a)[K], const int (&w)[K], const int (&d)[K],
-                                           int r, unsigned round_id, bool enq, LStats &ls) {
+                                           int r, bool enq, LStats &ls) {
   int pk[K];  // partner arcs, loaded while the atomics below are in flight
 #pragma unroll
   for (int k = 0; k < K; k++) pk[k] = d[k] > 0 ? __ldg(p.par + a[k]) : 0;
@@ -1433,9 +1434,9 @@ __device__ __forceinline__ void push_batch(const Params &p, const int (&a)[K], c
     if (d[k] > 0) {
       atomicAdd(p.res + pk[k], d[k]);
       ls.pushes++;
-      if (enq && !is_term(p, w[k]) && old[k] + d[k] > 0) cand |= 1u << k;
+      if (enq && old[k] <= 0 && old[k] + d[k] > 0 && !is_term(p, w[k])) cand |= 1u << k;
     }
-  if (cand) enqueue_batch<K>(p, w, cand, r, round_id);
+  if (cand) enqueue_batch<K>(p, w, cand, r);
 }
 
 // Adjacency bound of the register-resident thread discharge below.
@@ -1452,7 +1453,7 @@ constexpr int kSmallMax = 8;
 // the exact distance for a while; labels only steer the pushes -- dead
 // vertices and termination are decided by the exact BFS of each relabel.
 __device__ __forceinline__ void discharge_small(const Params &p, int v, int beg, int deg, long long ex0, int h, int r,
-                                unsigned round_id, bool enq, LStats &ls) {
+                                                bool enq, LStats &ls) {
   int rr[kSmallMax], w[kSmallMax], hw[kSmallMax];
 #pragma unroll
   for (int k = 0; k < kSmallMax; k++) {
@@ -1496,7 +1497,7 @@ __device__ __forceinline__ void discharge_small(const Params &p, int v, int beg,
         atomicAdd(p.res + pk[k], dd[k]);
         rr[k] -= dd[k];
         ls.pushes++;
-        if (enq && !is_term(p, w[k]) && old[k] + dd[k] > 0) cand |= 1u << k;
+        if (enq && old[k] <= 0 && old[k] + dd[k] > 0 && !is_term(p, w[k])) cand |= 1u << k;
       }
     ex = left;
     if (ex > 0) {  // every admissible arc is saturated: relabel
@@ -1509,14 +1510,15 @@ __device__ __forceinline__ void discharge_small(const Params &p, int v, int beg,
       ls.relabels++;
     }
   }
-  if (ex0 != ex) atomic_add_ll(p.excess + v, ex - ex0);
+  // what is left, with what arrived meanwhile
+  if (ex0 != ex) ex = atomic_add_ll(p.excess + v, ex - ex0) + (ex - ex0);
   if (enq && ex > 0 && h < p.n) cand |= 1u << kSmallMax;
   if (!cand) return;
   int x[kSmallMax + 1];
 #pragma unroll
   for (int k = 0; k < kSmallMax; k++) x[k] = w[k];
   x[kSmallMax] = v;
-  enqueue_batch<kSmallMax + 1>(p, x, cand, r, round_id);
+  enqueue_batch<kSmallMax + 1>(p, x, cand, r);
 }
 
 // Discharge of a non-hub v by a lane or a tile: up to `cycles` rounds of
@@ -1534,8 +1536,7 @@ __device__ __forceinline__ void discharge_small(const Params &p, int v, int beg,
 // raise heights, so a pass-2 arc that lost admissibility is skipped and the
 // round is retried instead of relabelled.
 template <class G>
-__device__ __forceinline__ void discharge(G &g, const Params &p, int v, int r, unsigned round_id, bool enq, LStats &ls,
-                          int *seen) {
+__device__ __forceinline__ void discharge(G &g, const Params &p, int v, int r, bool enq, LStats &ls, int *seen) {
   long long ex0;
   int h;
   // one read, broadcast: concurrent pushes may change excess[v] meanwhile
@@ -1562,7 +1563,7 @@ __device__ __forceinline__ void discharge(G &g, const Params &p, int v, int r, u
   constexpr int S = G::size();
   if constexpr (S == 1) {
     if (end - beg <= kSmallMax) {
-      discharge_small(p, v, beg, end - beg, ex0, h, r, round_id, enq, ls);
+      discharge_small(p, v, beg, end - beg, ex0, h, r, enq, ls);
       return;
     }
   }
@@ -1586,7 +1587,7 @@ __device__ __forceinline__ void discharge(G &g, const Params &p, int v, int r, u
         long long left = ex - pre;
         d = left <= 0 ? 0 : (left < rr ? (int)left : rr);
       }
-      if (d > 0) push_arc(p, a, w, d, r, round_id, enq, ls);
+      if (d > 0) push_arc(p, a, w, d, r, enq, ls);
       ex -= (tot < ex ? tot : ex);
       if (ex > 0) {
         const int mh = g.min_all(rr > 0 && !(adm && d == rr) ? hw : INT_MAX);
@@ -1647,7 +1648,7 @@ __device__ __forceinline__ void discharge(G &g, const Params &p, int v, int r, u
           done += dd[k];
         }
       }
-      push_batch<kPushBatch>(p, aa, w, dd, r, round_id, enq, ls);
+      push_batch<kPushBatch>(p, aa, w, dd, r, enq, ls);
     }
     const long long moved = g.sum_all(done);
     ex -= moved;
@@ -1661,8 +1662,8 @@ __device__ __forceinline__ void discharge(G &g, const Params &p, int v, int r, u
     }
   }
   if (g.rank() == 0) {
-    if (ex0 != ex) atomic_add_ll(p.excess + v, ex - ex0);
-    if (enq && ex > 0 && h < p.n) enqueue(p, r, round_id, v);
+    if (ex0 != ex) ex = atomic_add_ll(p.excess + v, ex - ex0) + (ex - ex0);
+    if (enq && ex > 0 && h < p.n) enqueue(p, r, v);
   }
 }
 
@@ -1701,8 +1702,7 @@ __device__ __forceinline__ RoundIn round_inputs(const Params &p, const Ctrl *c, 
 // chunk sums its admissible residual, adds its minimum non-admissible head
 // height to the hub's, and pushes its share of the hub's excess.
 template <int TILE>
-__device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int r, unsigned round_id, unsigned gepoch,
-                                         LStats &ls, bool dph) {
+__device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int r, unsigned gepoch, LStats &ls, bool dph) {
   Ctrl *c = p.ctrl;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const bool topo = p.variant == DMF_VARIANT_TOPO && !dph;
@@ -1800,7 +1800,7 @@ __device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int
               done += dd[k];
             }
           }
-          push_batch<kBatch>(p, aa, w, dd, r, round_id, !topo, ls);
+          push_batch<kBatch>(p, aa, w, dd, r, !topo, ls);
           moved = wg.sum_all(done);
           if (wg.rank() == 0 && moved) atomic_add_ll(p.hc_moved + hid, moved);
         }
@@ -1818,7 +1818,7 @@ __device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int
   // topology rounds sweep every vertex: only those with excess need a look
   for_tiered<TILE>(
       p, ls, in.nlist, in.nn,
-      [&](auto &g, int v) { discharge(g, p, v, r, round_id, !topo, ls, topo ? &seen : nullptr); },
+      [&](auto &g, int v) { discharge(g, p, v, r, !topo, ls, topo ? &seen : nullptr); },
       [&](int v) { return !topo || (__ldcg(p.excess + v) > 0 && inst_on(p, v)); });
   if (topo) block_add_int(1, &c->seen[r % 3], seen);
   sink_flush(p, ls);
@@ -1828,8 +1828,7 @@ __device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int
 // its excess; when all of the hub's admissible residual was pushed and excess is
 // left, the hub is relabelled to 1 + the minimum non-admissible height; a hub
 // with excess left is queued for the next round.  The hub's totals are reset.
-__device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int r, unsigned round_id, LStats &ls,
-                                         bool dph) {
+__device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int r, LStats &ls, bool dph) {
   const int nt = gridDim.x * blockDim.x;
   const bool topo = p.variant == DMF_VARIANT_TOPO && !dph;
   int seen = 0;
@@ -1858,7 +1857,7 @@ __device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int
       p.height[v] = h;
       ls.relabels++;
     }
-    if (!topo && ex > 0 && h < p.n) enqueue(p, r, round_id, v);
+    if (!topo && ex > 0 && h < p.n) enqueue(p, r, v);
   }
   if (topo) block_add_int(0, &p.ctrl->seen[r % 3], seen);
 }
@@ -2238,6 +2237,9 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   }
 
   unsigned round_id = p.round_base;
+  // Deep graphs: once a relabel has gone kDeepLevels levels, it and the rest of
+  // the solve use the barrier-free phases, where the grid can own every vertex.
+  const bool deep_ok = p.adaptive && p.interval <= kDeepLevels && async_fits(p.n);
 
   // ---- local repair inside the kept dead set ------------------------------------
   bool revive = true;  // the first global relabel revives every vertex
@@ -2291,7 +2293,9 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
           const Slot *in = slot_in();
           if (L > 0) scanned += in->arcs;
           if (in->q + in->hq == 0) break;
-          if (scanned > budget) {
+          // (a deep graph is better off with one complete barrier-free relabel
+          // than with a revival of as many phases as it has levels)
+          if (scanned > budget || (deep_ok && L >= kReviveLevels && p.variant != DMF_VARIANT_PP)) {
             revive = true;
             break;
           }
@@ -2322,6 +2326,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
         const int F = in->q + in->hq;
         reached += in->cnt;
         if (F == 0 || P == 0 || reached == P) break;
+        if (deep_ok && L >= kDeepLevels) break;  // the rest waits for the general solve
         kind = TR_PP_BFS;
         items = in->q;
         hubitems = in->hq;
@@ -2351,9 +2356,6 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   const bool cut_only = p.mode == MODE_CUT;
   const bool listed = !revive && p.lst;  // the live list holds for this solve
   const bool topo = p.variant == DMF_VARIANT_TOPO;
-  // Deep graphs: once a relabel has gone kDeepLevels levels, it and the rest of
-  // the solve use the barrier-free phases, where the grid can own every vertex.
-  const bool deep_ok = p.adaptive && p.interval <= kDeepLevels && async_fits(p.n);
   bool deep = false;
   for (int it = 0;; it++) {
     if (it >= p.max_iters) {
@@ -2443,11 +2445,11 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
       kind = TR_PUSH;
       items = in.nn;
       hubitems = in.nh;
-      ph_push1<TILE>(p, in, r, round_id, p.relabel_base + it, ls, false);
+      ph_push1<TILE>(p, in, r, p.relabel_base + it, ls, false);
       if (!next()) return;
       if (in.nh > 0) {
         kind = TR_PUSH_HUB_FINISH;
-        ph_push3(p, in, r, round_id, ls, false);
+        ph_push3(p, in, r, ls, false);
         if (!next()) return;
       }
       if (lead) {
