@@ -194,8 +194,12 @@ __device__ __forceinline__ void acc_flush() {
     const unsigned long long x = acc.v[i];
     if (x) {
       const unsigned long long to = (unsigned long long)acc.to[i];
-      if (to & 1) atomicAdd((int *)(to & ~1ull), (int)x);
-      else atomicAdd((unsigned long long *)to, x);
+      // with the old value read back: in a grid of one block the same warp reads
+      // the control block next, without a fence
+      unsigned long long old;
+      if (to & 1) old = (unsigned long long)atomicAdd((int *)(to & ~1ull), (int)x);
+      else old = atomicAdd((unsigned long long *)to, x);
+      asm volatile("" ::"l"(old) : "memory");
       acc.v[i] = 0;
     }
   }
@@ -228,7 +232,7 @@ __device__ __forceinline__ bool grid_barrier(Ctrl *c, Ctrl *snap, unsigned long 
   if (threadIdx.x < 32) {
     acc_flush();
     __syncwarp();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && gridDim.x > 1) {  // one block: the block barriers are enough
       const unsigned nb = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
       const unsigned old = atom_add_release_u32(&c->bar_count, nb);
       unsigned long long t0 = 0;

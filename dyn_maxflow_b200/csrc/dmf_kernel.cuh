@@ -670,13 +670,17 @@ __device__ __forceinline__ void for_vertices(const Params &p, F &&f) {
 // (nearly all of them when a batch keeps the dead set) costs that load and a
 // vote.  Other windows are walked like for_vertices (v = window + 32 j + lane,
 // coalesced), the flags coming again from L2.  Calls with an instance mask
-// take the plain per-vertex walk.
+// take the plain per-vertex walk, and so do graphs of up to kPlainSweep vertices
+// per thread: there 16 vertices a lane would leave most warps without a window
+// (seed passes of a static solve 59 -> 25 us at R-MAT 14, finalize 18 -> 5 at 138 k
+// vertices).
 constexpr int kWindow = 512;
+constexpr int kPlainSweep = 8;
 
 template <int U, class F>
 __device__ __forceinline__ int for_live_vertices(const Params &p, F &&f) {
   int seen = 0;
-  if (p.inst_active) {
+  if (p.inst_active || p.n <= kPlainSweep * (int)(gridDim.x * blockDim.x)) {
     for_vertices<U>(p, [&](int v, bool is_dead) {
       if (is_dead) return;
       seen++;
@@ -725,13 +729,14 @@ __device__ __forceinline__ int for_live_vertices(const Params &p, F &&f) {
 // short; entries that died since are skipped by their flag.  With ~400 live
 // vertices of 1 M the walk takes one dependent load more than an empty phase
 // where the sweep reads every flag (seed pass 9 -> 4 us at R-MAT 20, 16 -> 4 at
-// R-MAT 22); past a quarter of the vertices the sweep's coalesced reads win.
+// R-MAT 22); past a quarter of the vertices the sweep's coalesced reads win,
+// unless every thread has at most one entry.
 template <int U, class F>
 __device__ __forceinline__ int for_live(const Params &p, bool listed, F &&f) {
   if (listed) {
     const int cnt = __ldcg(p.lst);
-    if (4ll * cnt < p.n) {
-      const int nt = gridDim.x * blockDim.x;
+    const int nt = gridDim.x * blockDim.x;
+    if (4ll * cnt < p.n || cnt <= nt) {
       int seen = 0;
       for (int i = spread_thread(); i < cnt; i += nt) {
         const int v = __ldcg(p.lq + i);
@@ -988,7 +993,7 @@ __device__ __forceinline__ void ph_bfs_bu(const Params &p, Slot *out, int L, LSt
     }
   }
   // eight lanes a vertex at most: most rows have a hit in their first 64 arcs,
-  // and a warp keeps four rows in flight (R-MAT 20: level 134 -> 98 us)
+  // and a warp keeps four rows in flight (R-MAT 20: level 134 -> 105 us)
   constexpr int BT = TILE < 8 ? TILE : 8;
   for_tiered<BT>(p, ls, nullptr, p.n, [&](auto &g, int v) {
     if (__ldcg(p.height + v) != UNV) return;  // only v's group writes it in this phase
@@ -1162,6 +1167,61 @@ __device__ __forceinline__ long long pull_lower(const Params &p, cg::thread_bloc
   return (long long)warp_sum_u64(0xffffffffu, (unsigned long long)take);
 }
 
+// Pass 0 on a stretch of a long row: kPullBatch arcs a lane, their loads in
+// flight together, one prefix sum over the lanes' totals, exact claims as in
+// pull_excess.  Returns what the warp moved.
+constexpr int kPullBatch = 4;
+
+__device__ __forceinline__ long long pull_stretch(const Params &p, cg::thread_block_tile<32> &warp, int a0, int end,
+                                                  long long need, LStats &ls) {
+  int x[kPullBatch], pa[kPullBatch];
+  long long cand[kPullBatch], tot = 0;
+#pragma unroll
+  for (int j = 0; j < kPullBatch; j++) {
+    const int a = a0 + 32 * j;
+    x[j] = a < end ? __ldg(p.adj + a) : -1;
+    pa[j] = a < end ? __ldg(p.par + a) : 0;
+  }
+#pragma unroll
+  for (int j = 0; j < kPullBatch; j++) {
+    cand[j] = 0;
+    if (x[j] < 0) continue;
+    ls.arcs++;
+    const int r = __ldcg(p.res + pa[j]);
+    const bool dx = __ldcg(p.dead + x[j]) != 0;
+    const long long ex = __ldcg(p.excess + x[j]);
+    if (r > 0 && dx && ex > 0 && !is_term(p, x[j])) cand[j] = ex < r ? ex : (long long)r;
+  }
+#pragma unroll
+  for (int j = 0; j < kPullBatch; j++) tot += cand[j];
+  if (!__any_sync(0xffffffffu, tot > 0)) return 0;
+  long long left = need - cg::exclusive_scan(warp, tot, cg::plus<long long>());
+  long long got = 0;
+  long long take[kPullBatch], old[kPullBatch];
+#pragma unroll
+  for (int j = 0; j < kPullBatch; j++) {
+    take[j] = left <= 0 ? 0 : (left < cand[j] ? left : cand[j]);
+    left -= take[j];
+    if (take[j] > 0) old[j] = atomic_add_ll(p.excess + x[j], -take[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < kPullBatch; j++) {
+    if (take[j] <= 0) continue;
+    if (old[j] < take[j]) {  // another puller was first: hand back what it took
+      const long long back = take[j] - (old[j] > 0 ? old[j] : 0);
+      atomic_add_ll(p.excess + x[j], back);
+      take[j] -= back;
+    }
+    if (take[j] > 0) {
+      atomicSub(p.res + pa[j], (int)take[j]);
+      atomicAdd(p.res + a0 + 32 * j, (int)take[j]);
+      got += take[j];
+      ls.pushes++;
+    }
+  }
+  return (long long)warp_sum_u64(0xffffffffu, (unsigned long long)got);
+}
+
 // Warps first_warp, first_warp + nwarps, ... take the list's deficits; the next
 // round's list is appended behind *ntail.  seed: the list is the candidates
 // themselves (a list of at most a candidate per warp spares the seed phase);
@@ -1202,35 +1262,38 @@ __device__ __forceinline__ void ph_dead_pull(const Params &p, const int *list, i
         got += mv;
       }
     } else {
-      // two steps' loads in flight at a time, starting at the row's cursor:
-      // where the last pass 0 of this deficit was satisfied.  A hub deficit
-      // that comes back batch after batch would otherwise rescan the in-arcs
-      // whose suppliers it drained earlier (at R-MAT 24 the longest item of a
-      // round, a hub of 60-165 k in-arcs, grew from 90 us to 550 us over 16
-      // batches, and every round waits for it).
+      // Starting at the row's cursor: where the last pass 0 of this deficit was
+      // satisfied.  A hub deficit that comes back batch after batch would
+      // otherwise rescan the in-arcs whose suppliers it drained earlier (at
+      // R-MAT 24 the longest item of a round, a hub of 60-165 k in-arcs, grew
+      // from 90 us to 550 us over 16 batches, and every round waits for it).
+      // Pass 0 takes 128 arcs at a time, pass 1 two steps of 32.
       const int deg = end - beg;
       int cur = p.pcur ? __ldcg(p.pcur + y) : 0;
       cur = (cur < 0 || cur >= deg) ? 0 : (cur & ~31);
       int stop = -1;
-      for (int pass = 0; pass < 2 && need > 0; pass++) {
-        for (int seg = 0; seg < 2 && need > 0; seg++) {
-          const int sb = seg == 0 ? beg + cur : beg, se = seg == 0 ? end : beg + cur;
-          for (int a0 = sb; a0 < se && need > 0; a0 += 64) {
-            PullArc q0 = pull_load(p, a0 + lane, se);
-            PullArc q1 = pull_load(p, a0 + 32 + lane, se);
-            ls.arcs += (q0.x >= 0) + (q1.x >= 0);
-            long long mv = pass == 0 ? pull_excess(p, warp, q0, need, ls)
-                                     : pull_lower(p, warp, q0, need, hy, hmin, nxt, ntail, round_id, ls);
+      for (int seg = 0; seg < 2 && need > 0; seg++) {
+        const int sb = seg == 0 ? beg + cur : beg, se = seg == 0 ? end : beg + cur;
+        for (int a0 = sb; a0 < se && need > 0; a0 += 32 * kPullBatch) {
+          const long long mv = pull_stretch(p, warp, a0 + lane, se, need, ls);
+          need -= mv;
+          got += mv;
+          if (need <= 0) stop = a0;
+        }
+      }
+      for (int seg = 0; seg < 2 && need > 0; seg++) {
+        const int sb = seg == 0 ? beg + cur : beg, se = seg == 0 ? end : beg + cur;
+        for (int a0 = sb; a0 < se && need > 0; a0 += 64) {
+          PullArc q0 = pull_load(p, a0 + lane, se);
+          PullArc q1 = pull_load(p, a0 + 32 + lane, se);
+          ls.arcs += (q0.x >= 0) + (q1.x >= 0);
+          long long mv = pull_lower(p, warp, q0, need, hy, hmin, nxt, ntail, round_id, ls);
+          need -= mv;
+          got += mv;
+          if (need > 0 && a0 + 32 < se) {
+            mv = pull_lower(p, warp, q1, need, hy, hmin, nxt, ntail, round_id, ls);
             need -= mv;
             got += mv;
-            if (pass == 0 && need <= 0) stop = a0;
-            if (need > 0 && a0 + 32 < se) {
-              mv = pass == 0 ? pull_excess(p, warp, q1, need, ls)
-                             : pull_lower(p, warp, q1, need, hy, hmin, nxt, ntail, round_id, ls);
-              need -= mv;
-              got += mv;
-              if (pass == 0 && need <= 0) stop = a0 + 32;
-            }
           }
         }
       }
@@ -1367,7 +1430,7 @@ __device__ __forceinline__ void ph_dead_revive(const Params &p, const Slot *in, 
 // when it raised the excess from zero or below to above.  The excess word orders
 // these: within a round it falls once at most, so only one of them sees the
 // change.  (A stamp exchanged by every push put a second returning atomic, on
-// the busiest hubs' words, behind the first: R-MAT 20 push round 83 -> 58 us.)
+// the busiest hubs' words, behind the first: R-MAT 20 push round 83 -> 75.5 us.)
 __device__ __forceinline__ void enqueue(const Params &p, int r, int v) {
   if (deg_of(p, v) > p.hub_deg) append_hub(p, p.wh[r & 1], &p.ctrl->whtail[r % 3], v);
   else append(p.wq[r & 1], &p.ctrl->wtail[r % 3], v);
@@ -1744,7 +1807,7 @@ __device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int
     // A warp's lanes first read the headers of its next 32 chunks (hub, label,
     // excess, mark: three dependent loads, once for all of them instead of once
     // per chunk); the chunks that have something to scan are then done in turn.
-    // R-MAT 20: 36,000 chunks a round, push round 75.5 -> 58 us.
+    // R-MAT 20: 36,000 chunks a round, push round 75.5 -> 70.6 us.
     TileGroup<32> wg;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int base = spread_group<32>(); base < in.nh; base += 32 * nwarps) {
@@ -1912,8 +1975,17 @@ __device__ __forceinline__ void ph_flow(const Params &p, bool listed) {
       acc += c;
     }
   };
+  const int nt = gridDim.x * blockDim.x;
   if (listed || !p.lst) {
     for_live<8>(p, listed, add);
+  } else if (p.n <= kPlainSweep * nt) {
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < p.n; v += nt) {
+      const bool d = __ldcg(p.dead + v) != 0;
+      p.inl[v] = d ? 0 : 1;
+      if (d) continue;
+      append(p.lq, p.lst, v);
+      if (inst_on(p, v)) add(v);
+    }
   } else {
     const int lane = threadIdx.x & 31;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;

@@ -260,6 +260,8 @@ void free_all(dmf_solver *sv) {
   sv->ev0 = sv->ev1 = nullptr;
 }
 
+constexpr int kTinyVertices = kBlock, kTinyArcs = 8 * kBlock;
+
 int choose_tile(const dmf_opts &o, int n, int m) {
   if (o.tile == 1 || o.tile == 2 || o.tile == 4) return 4;
   if (o.tile == 8 || o.tile == 16 || o.tile == 32) return o.tile;
@@ -292,6 +294,10 @@ int configure(dmf_solver *sv) {
   if (!coop || per_sm < 1) return fail(DMF_ERR_CUDA, "device does not support cooperative launch of the solver");
   sv->grid = per_sm * sms;
   if (sv->opts.grid_blocks > 0) sv->grid = std::min(sv->grid, sv->opts.grid_blocks);
+  // A graph that one block's threads cover has no use for a second block, and a
+  // grid of one needs no grid barrier (420 arcs: 82 -> 62 us a batch; 0.5 M arcs
+  // would lose: 90 us against 66).
+  if (sv->n <= kTinyVertices && sv->m <= kTinyArcs) sv->grid = 1;
   if (sv->opts.small_deg > 0) sv->small_deg = sv->opts.small_deg;
   else if (sv->opts.small_deg < 0) sv->small_deg = 0;  // no thread tier
   sv->block = kBlock;
