@@ -16,8 +16,8 @@
 // BFS levels after which a global relabel (and then the rest of the solve)
 // goes over to the barrier-free phases.  R-MAT graphs end within 10 levels:
 // there a level is real work and the worklists save polling every vertex.  A
-// graph that needs 24 levels will need hundreds of short phases.
-constexpr int kDeepLevels = 24;
+// graph that needs 16 levels (9 us each) will need hundreds of short phases.
+constexpr int kDeepLevels = 16;
 // Levels after which the partial revival of a batch gives up on such a graph.
 constexpr int kReviveLevels = 8;
 // Windows of 32 vertices per warp at most: bounds the vertices a graph may

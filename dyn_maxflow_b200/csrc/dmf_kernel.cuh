@@ -2343,7 +2343,10 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   const bool deep_ok = p.adaptive && p.interval <= kDeepLevels && async_fits(p.n);
 
   // ---- local repair inside the kept dead set ------------------------------------
-  bool revive = true;  // the first global relabel revives every vertex
+  // The first global relabel revives every vertex, unless the dead set of the
+  // last solve holds: in a batch that keeps it, and for the cut readout (no dead
+  // vertex reaches t or a deficit, so the cut is decided among the live ones).
+  bool revive = p.mode != MODE_CUT;
   if (p.mode == MODE_DYNAMIC && p.keep_dead) {
     revive = false;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;

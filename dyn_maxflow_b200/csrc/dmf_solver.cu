@@ -1023,12 +1023,13 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
   if (e == cudaSuccess) e = cudaEventCreate(&sv->ev1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(S);
   if (e != cudaSuccess) return cuda_fail(e, "solver upload");
-  // staging for an eighth of the arcs up front, up to 2^18 updates, and for 3%
-  // beyond that on the device (a call that has to grow it waits for the device
-  // and for the allocations: ms, at times tens of ms)
+  // Staging up front: on the device for an eighth of the arcs, up to 2^18 updates,
+  // and for 3% beyond that (a call that has to grow it waits for the device and
+  // for the allocation, up to tens of ms); pinned, which costs ms per MiB to
+  // allocate and only host batches use, for up to 2^14 updates.
   const size_t some = std::min<size_t>(M / 8, 1 << 18);
   if ((st = ensure_ubuf(sv, (int)std::max<size_t>({1024, some, M / 32})))) return st;
-  if ((st = ensure_host_ubuf(sv, (int)std::max<size_t>(1024, some)))) return st;
+  if ((st = ensure_host_ubuf(sv, (int)std::max<size_t>(1024, std::min<size_t>(M / 64, 1 << 14))))) return st;
   // sources (and, for batched instances, roles, instance ids, per-instance flows)
   {
     const std::vector<int> one(1, s);
@@ -1440,6 +1441,7 @@ int dmf_get_cut(dmf_solver *sv, uint8_t *sink_side) {
       int64_t f = sv->st.flow;
       resolve_ms(sv);
       dmf_stats keep = sv->st;
+      CK(cudaMemsetAsync(sv->side, 0, (size_t)sv->n, sv->stream), "clear cut");  // the relabel sets live vertices
       int st = run_mode(sv, MODE_CUT, 0, nullptr, nullptr, nullptr, nullptr, false);
       if (st) return st;
       sv->st = keep;
