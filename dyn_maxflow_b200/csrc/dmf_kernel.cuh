@@ -64,7 +64,7 @@ struct Params {
   const int *__restrict__ off;
   const int *__restrict__ adj;
   const int *__restrict__ par;
-  ArcSlot *atab;    // (tail, head) -> arc table with the per-arc batch stamps
+  ArcSlot *atab;    // (tail, head) -> arc table
   long long nslots;  // its slots
   int *cap;                  // capacities as a plain array (allocation-free static solve only)
   unsigned long long *capx;  // capacities of a solver: (epoch of the batch that set it << 32) | capacity
@@ -2523,8 +2523,9 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
       if (!next()) return;
       if (lead) c->st_levels += (unsigned long long)max(0, sc->adepth + 1 - L);
       if (sc->aact == 0 || cut_only) break;
-      // as long again as the relabel took: on the 256 x 256 grid half of that
-      // costs 27 ms a solve, the same 22 ms, twice 24 ms
+      // as long again as the relabel took: a solve of the 256 x 256 grid takes
+      // 16 ms so, 17 with 1.5 times that, 18 with twice, 21 with three times
+      // (half: 27 ms against 22 when a hop took 0.8 us)
       kind = TR_PUSH_ASYNC;
       items = sc->aact;
       ph_async_push(p, ash, lead ? globaltimer() - t_bfs : 0, ls);
