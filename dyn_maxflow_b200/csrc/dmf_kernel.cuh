@@ -928,11 +928,19 @@ __device__ __forceinline__ void ph_bfs_td(const Params &p, const Slot *in, Slot 
   const int nn = ld_vol(&in->q), nh = ld_vol(&in->hq);
   VisitAcc acc;
   const int lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int i = spread_group<32>(); i < nh; i += nwarps) {
+  // A short list (the sink's row, at the start of every relabel) is cut finer:
+  // half a chunk is one register batch, so its chain of loads runs once (R-MAT
+  // 20: 109 chunks of the sink, level 15.5 -> 11 us).
+  const int cut = 2 * nh <= nwarps ? 1 : 0;
+  for (int i = spread_group<32>(); i < nh << cut; i += nwarps) {
     int beg, end;
-    const int2 it = __ldcg(p.fh[cur] + i);
+    const int2 it = __ldcg(p.fh[cur] + (i >> cut));
     ItemTimer tm(p);
     chunk_range(p, it, beg, end);
+    if (cut) {
+      beg += (i & 1) * (kChunk / 2);
+      end = min(end, beg + kChunk / 2);
+    }
     td_range(p, out, nxt, beg + lane, end, 32, L, ls, acc);
     tm.done(ls, it.x);
   }
