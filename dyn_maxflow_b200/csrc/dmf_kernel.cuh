@@ -930,7 +930,7 @@ __device__ __forceinline__ void ph_bfs_td(const Params &p, const Slot *in, Slot 
   const int lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
   // A short list (the sink's row, at the start of every relabel) is cut finer:
   // half a chunk is one register batch, so its chain of loads runs once (R-MAT
-  // 20: 109 chunks of the sink, level 15.5 -> 11 us).
+  // 20: 109 chunks of the sink, level 15.5 -> 10.9 us).
   const int cut = 2 * nh <= nwarps ? 1 : 0;
   for (int i = spread_group<32>(); i < nh << cut; i += nwarps) {
     int beg, end;
