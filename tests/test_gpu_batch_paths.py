@@ -1,6 +1,9 @@
 """The one-pass lookup and claim of a batch, and the phases it lets a batch skip: rejected batches leave no trace
 (with and without the bound on capacities that allows the one pass), source arcs are the only ones a batch has to
-saturate, both arcs of a pair in one batch, and the live list over batches that kill and revive vertices."""
+saturate, both arcs of a pair in one batch, the live list over batches that kill and revive vertices, the ways to sweep
+it, and the sizes at which the staging of a host batch changes."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -100,3 +103,41 @@ def test_live_list_over_a_stream(dmf, oracle, scale, frac):
                 side = sv.cut()
                 tail = np.repeat(np.arange(g.num_nodes()), np.diff(index))
                 assert int(cur[(side[tail] == 0) & (side[adj] == 1)].sum()) == want
+
+
+# up to 8 vertices a thread are walked plainly, beyond that in windows of 512 (8192 vertices on 1 block of 512 threads)
+@pytest.mark.parametrize("blocks,scale", [(1, 12), (1, 13), (2, 13), (3, 14)])
+def test_sweeps_on_few_blocks(dmf, oracle, blocks, scale):
+    g, s, t = rmat(dmf, scale)
+    index, adj, w, par = g.arrays()
+    cur = w.copy()
+    with dmf.Solver(g, s, t) as sv:
+        o = dmf.Opts()
+        dmf._L.dmf_opts_default(ctypes.byref(o))
+        o.grid_blocks = blocks
+        dmf._check(dmf._L.dmf_solver_set_opts(sv._h, ctypes.byref(o)))
+        assert sv.static_maxflow() == oracle.dinic(g.num_nodes(), index, adj, cur, par, s, t)
+        for i, b in enumerate(dmf.gen_batches(g, 4, frac=0.1, p_inc=0.3, p_dec=0.3, p_ins=0.1, seed=blocks)):
+            apply_host(g, cur, b)
+            want = oracle.dinic(g.num_nodes(), index, adj, cur, par, s, t)
+            assert sv.apply_updates(*b) == want
+            certify(oracle, g, sv, s, t, want)
+            side = sv.cut()
+            tail = np.repeat(np.arange(g.num_nodes()), np.diff(index))
+            assert int(cur[(side[tail] == 0) & (side[adj] == 1)].sum()) == want
+
+
+# where the staging of a host batch changes: copied by one thread, by several, sent to the device in pieces
+@pytest.mark.parametrize("k", [16384, 16385, 262144, 262145])
+def test_staging_sizes(dmf, k):
+    torch = pytest.importorskip("torch")
+    g, s, t = rmat(dmf, 16)
+    rng = np.random.default_rng(k)
+    pick = rng.permutation(g.num_edges())[:k]
+    src, dst = arcs_of(g, pick)
+    to = rng.integers(0, 2000, k).astype(np.int32)
+    with dmf.Solver(g, s, t) as sv, dmf.Solver(g, s, t) as other:
+        sv.static_maxflow()
+        d = [torch.from_numpy(x).cuda() for x in (src, dst, to)]
+        assert sv.apply_updates(src, dst, to) == other.recompute_device(*(x.data_ptr() for x in d), k)
+        assert np.array_equal(sv.state()[0], other.state()[0])
