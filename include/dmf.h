@@ -230,7 +230,8 @@ int dmf_stats_get(const dmf_solver *sv, dmf_stats *st);
 /* Phase timeline of the last solve call (needs DMF_FLAG_TRACE): entry 0 is the
  * kernel start (kind 0); entry i > 0 is the end of a phase of kind kinds[i] at
  * t_us[i] microseconds after the start.  Kinds: 1 init residuals, 2 source
- * saturation, 3 arc lookup, 4 capacity apply, 5 over-capacity repair, 6 cut
+ * saturation, 3 arc lookup with the capacity claim and apply, 4 claim and
+ * apply by themselves (capacities above 2^30-1), 5 over-capacity repair, 6 cut
  * saturation, 7 BFS seeds, 8 BFS top-down level, 9 BFS bottom-up level,
  * 10 BFS finalize, 11 push round, 12 flow readout, 13/14 hub push rounds,
  * 15-18 push-pull phase 1, 19 reopen, 20 dead-set pull seeding, 21 pull round,
