@@ -36,17 +36,6 @@ struct AsyncShared {
   int stop;
 };
 
-__device__ __forceinline__ int ld_rlx(const int *p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ long long ld_rlx(const long long *p) {
-  long long v;
-  asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
 // The windows of a warp: block b owns `per` consecutive windows, warp i of it
 // windows i, i + warps, ...
 struct AsyncOwn {
@@ -106,7 +95,13 @@ __device__ __forceinline__ void async_wake(AsyncShared &sh, AsyncIdle &st, int *
     if ((threadIdx.x & 31) == 0 && atomicSub(&sh.idle_warps, 1) == (int)(blockDim.x >> 5)) atomicSub(idle_blocks, 1);
   }
 }
-__device__ __forceinline__ bool async_stopped(const AsyncShared &sh) { return *(const volatile int *)&sh.stop != 0; }
+// Whether the warp leaves the phase.  Every lane calls it, and the answer is the
+// warp's: another warp (or thread 0 of this one, just before) may set the word
+// between two lanes' reads, and a lane that left by itself would wait at
+// async_end's block barrier for lanes that wait for it in the next poll's vote.
+__device__ __forceinline__ bool async_stopped(const AsyncShared &sh) {
+  return __any_sync(0xffffffffu, *(const volatile int *)&sh.stop != 0);
+}
 
 // Every warp has left: a block that stopped while one of its warps had just woken
 // is counted as idle again, or the others would wait for it.

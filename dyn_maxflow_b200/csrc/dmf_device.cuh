@@ -9,6 +9,8 @@
 #include <cooperative_groups/reduce.h>
 #include <cooperative_groups/scan.h>
 
+#include "dmf_ptx.cuh"
+
 namespace dmfd {
 
 namespace cg = cooperative_groups;
@@ -94,31 +96,8 @@ struct HostResult {
 };
 
 // ---- memory helpers ---------------------------------------------------------
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned atom_add_release_u32(unsigned *p, unsigned x) {
-  unsigned v;
-  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(x) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned *p, unsigned x) {
-  unsigned v;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(x) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_sys_u32(unsigned *p, unsigned x) {
-  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
-}
 __device__ __forceinline__ int ld_vol(const int *p) { return *(const volatile int *)p; }
 __device__ __forceinline__ long long ld_vol(const long long *p) { return *(const volatile long long *)p; }
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 __device__ __forceinline__ long long atomic_add_ll(long long *p, long long v) {
   return (long long)atomicAdd((unsigned long long *)p, (unsigned long long)v);
 }
@@ -129,11 +108,6 @@ __device__ __forceinline__ long long atomic_add_ll(long long *p, long long v) {
 // every step of a scan, and partial warps are the rule here (a BFS level or a
 // push round of a few hundred vertices).  A phase is bound by the instructions
 // of its slowest warp, so these lengths matter more than the arithmetic.
-__device__ __forceinline__ unsigned lanemask_lt() {
-  unsigned m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
 
 // Sum of v over the lanes of `mask` (every one of them must call it), modulo
 // 2^64: three redux.sync over 24-, 24- and 16-bit pieces, whose 32-lane sums
@@ -199,7 +173,7 @@ __device__ __forceinline__ void acc_flush() {
       unsigned long long old;
       if (to & 1) old = (unsigned long long)atomicAdd((int *)(to & ~1ull), (int)x);
       else old = atomicAdd((unsigned long long *)to, x);
-      asm volatile("" ::"l"(old) : "memory");
+      keep_u64(old);
       acc.v[i] = 0;
     }
   }
