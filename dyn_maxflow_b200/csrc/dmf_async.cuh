@@ -466,36 +466,12 @@ __device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh,
   }
 }
 
-__device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, unsigned long long budget_ns,
-                                              LStats &ls) {
+// The same for a warp of several windows.
+__device__ __forceinline__ void async_push_loop(const Params &p, AsyncShared &sh, const AsyncOwn &own, unsigned live,
+                                                bool lead, unsigned long long t0, unsigned long long budget_ns,
+                                                LStats &ls) {
   Ctrl *c = p.ctrl;
-  const AsyncOwn own = async_own(p.n);
   const int lane = threadIdx.x & 31;
-  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-  unsigned long long t0 = 0;
-  if (lead) {
-    t0 = globaltimer();
-    c->pos_count = 0;
-    c->unexplored = 0;
-  }
-  async_begin(sh);
-  // a dead vertex's parked excess is not polled
-  unsigned live = 0;
-  for (int j = 0; j < own.count; j++) {
-    const int v = own.first + j * own.step + lane;
-    if (v < p.n && !__ldcg(p.dead + v) && !is_term(p, v) && inst_on(p, v)) live |= 1u << j;
-  }
-  if (own.count <= 1) {
-    const int v = own.first + lane;
-    const int deg = live & 1 ? deg_of(p, v) : 0;
-    if (__any_sync(0xffffffffu, deg > 4 && deg <= kSmallMax))
-      async_push_one<kSmallMax>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
-    else
-      async_push_one<4>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
-    async_end(sh, &c->aidle[1]);
-    sink_flush(p, ls);
-    return;
-  }
   TileGroup<32> wg;
   AsyncIdle st;
   for (int poll = 0;; poll++) {
@@ -545,6 +521,39 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
     } else if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) {
       break;
     }
+  }
+}
+
+__device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, unsigned long long budget_ns,
+                                              LStats &ls) {
+  Ctrl *c = p.ctrl;
+  const AsyncOwn own = async_own(p.n);
+  const int lane = threadIdx.x & 31;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  unsigned long long t0 = 0;
+  if (lead) {
+    t0 = globaltimer();
+    c->pos_count = 0;
+    c->unexplored = 0;
+  }
+  async_begin(sh);
+  // a dead vertex's parked excess is not polled
+  unsigned live = 0;
+  for (int j = 0; j < own.count; j++) {
+    const int v = own.first + j * own.step + lane;
+    if (v < p.n && !__ldcg(p.dead + v) && !is_term(p, v) && inst_on(p, v)) live |= 1u << j;
+  }
+  // The warps of a block may own different numbers of windows: they part here and
+  // meet again before the block barrier.
+  if (own.count <= 1) {
+    const int v = own.first + lane;
+    const int deg = live & 1 ? deg_of(p, v) : 0;
+    if (__any_sync(0xffffffffu, deg > 4 && deg <= kSmallMax))
+      async_push_one<kSmallMax>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
+    else
+      async_push_one<4>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
+  } else {
+    async_push_loop(p, sh, own, live, lead, t0, budget_ns, ls);
   }
   async_end(sh, &c->aidle[1]);
   sink_flush(p, ls);

@@ -51,9 +51,9 @@ def solve(kernel_main, oracle, tmp_path, n, width, blocks, warps, variant):
     return run(kernel_main, "solve", path, blocks, 32 * warps, variant), want
 
 
-# deep graphs: every warp one window of 32 vertices, some none, two, the most a warp can own
-@pytest.mark.parametrize("n,width,blocks,warps", [(64, 1, 1, 2), (64, 2, 2, 2), (30, 1, 1, 2), (97, 2, 1, 2),
-                                                  (256, 4, 1, 2)])
+# deep graphs: every warp one window of 32 vertices, some none, some more than others, the most a warp can own
+@pytest.mark.parametrize("n,width,blocks,warps", [(64, 1, 1, 2), (64, 2, 2, 2), (30, 1, 1, 2), (96, 1, 1, 2),
+                                                  (97, 2, 1, 2), (160, 3, 2, 2), (200, 2, 1, 4), (256, 4, 1, 2)])
 def test_deep_solve_stays_together(kernel_main, oracle, tmp_path, n, width, blocks, warps):
     got, want = solve(kernel_main, oracle, tmp_path, n, width, blocks, warps, 0)
     assert [x[0] for x in got] == want
