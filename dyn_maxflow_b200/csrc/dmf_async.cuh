@@ -27,7 +27,8 @@ constexpr int kAsyncWin = 4;
 // takes to become visible, so that a wave crossing from one block to another
 // does not find every block idle.
 constexpr int kQuietPolls = 8;
-// Polls per phase at most (bounds the loop; a phase is far shorter).
+// Polls of a block's first warp in a phase at most (bounds the loop, whatever
+// the polls find; a phase is far shorter).
 constexpr int kMaxPolls = 1 << 20;
 
 struct AsyncShared {
@@ -61,10 +62,10 @@ __device__ __forceinline__ bool async_fits(int n) {
 }
 
 // Quiescence: a warp is idle after kQuietPolls polls without work, a block when
-// all its warps are, and the phase ends once every block is idle (or *stop is
-// set).  This may end a phase too early (work in flight to an idle block); the
-// relabel checks its labels after a barrier, and a push phase may end at any
-// time.  One poll of the grid-wide words per block and 8 polls.
+// all its warps are, and the phase ends once every block is idle (or a limit of
+// async_look is reached).  This may end a phase too early (work in flight to an
+// idle block); the relabel checks its labels after a barrier, and a push phase
+// may end at any time.
 struct AsyncIdle {
   int quiet = 0;
   bool idle = false;
@@ -78,12 +79,14 @@ __device__ __forceinline__ void async_begin(AsyncShared &sh) {
   __syncthreads();
 }
 
-// The block's look at the phase's stop word, every 8th poll whatever the polls
+// The block's look at the limits of the phase, every 8th poll whatever the polls
 // find: a warp that finds work at every other poll (excess that goes to and fro
-// between two windows until its labels reach n) would else never look.
-__device__ __forceinline__ void async_look(AsyncShared &sh, int poll, const int *stop, const int *err) {
-  if (threadIdx.x == 0 && (poll & 7) == 7 && (ld_rlx(stop) || ld_rlx(err) || poll >= kMaxPolls))
-    *(volatile int *)&sh.stop = 1;
+// between two windows until its labels reach n) would else never look.  Every
+// block looks for itself: the block that set the deadline may have left already.
+__device__ __forceinline__ void async_look(const Params &p, AsyncShared &sh, int poll, bool timed) {
+  if (threadIdx.x != 0 || (poll & 7) != 7) return;
+  const unsigned long long end = timed ? ld_rlx(&p.ctrl->adeadline) : 0;
+  if (ld_rlx(&p.ctrl->err) || poll >= kMaxPolls || (end && globaltimer() > end)) *(volatile int *)&sh.stop = 1;
 }
 
 // A warp that found work; called before it does it, so that a long piece of work
@@ -111,18 +114,16 @@ __device__ __forceinline__ void async_end(AsyncShared &sh, int *idle_blocks) {
 }
 
 // A warp whose last poll found nothing; true: leave the phase.  The block's
-// first warp looks at the grid-wide words.  The SM's warps share its issue
+// first warp looks at the number of idle blocks.  The SM's warps share its issue
 // slots, so a poll is kept short and a warp without vertices sleeps.
-__device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool owner, int poll, int *idle_blocks,
-                                            const int *stop, const int *err) {
+__device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool owner, int *idle_blocks) {
   if (++st.quiet < kQuietPolls && owner) return false;
   if (!st.idle) {
     st.idle = true;
     if ((threadIdx.x & 31) == 0 && atomicAdd(&sh.idle_warps, 1) == (int)(blockDim.x >> 5) - 1)
       atomicAdd(idle_blocks, 1);
   }
-  if (threadIdx.x == 0 && (st.quiet & 3) == 0 &&
-      (ld_rlx(idle_blocks) >= (int)gridDim.x || ld_rlx(stop) || ld_rlx(err) || poll >= kMaxPolls))
+  if (threadIdx.x == 0 && (st.quiet & 3) == 0 && ld_rlx(idle_blocks) >= (int)gridDim.x)
     *(volatile int *)&sh.stop = 1;
   if (!owner) __nanosleep(200);
   return async_stopped(sh);
@@ -193,8 +194,9 @@ __device__ __forceinline__ void async_bfs_one(const Params &p, AsyncShared &sh, 
   for (int poll = 0;; poll++) {
     const int h = mine ? ld_rlx(p.height + v) : INT_MAX;
     const bool need = h < scan;
+    async_look(p, sh, poll, false);
     if (!__any_sync(0xffffffffu, need)) {
-      if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[0], &c->astop, &c->err)) break;
+      if (async_quiet(sh, st, own.count > 0, &c->aidle[0])) break;
       continue;
     }
     async_wake(sh, st, &c->aidle[0]);
@@ -266,8 +268,9 @@ __device__ __forceinline__ void async_bfs_loop(const Params &p, AsyncShared &sh,
     bool need_any = false;
 #pragma unroll
     for (int j = 0; j < W; j++) need_any |= h[j] < scan[j];
+    async_look(p, sh, poll, false);
     if (!__any_sync(0xffffffffu, need_any)) {
-      if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[0], &c->astop, &c->err)) break;
+      if (async_quiet(sh, st, own.count > 0, &c->aidle[0])) break;
       continue;
     }
     async_wake(sh, st, &c->aidle[0]);
@@ -302,7 +305,7 @@ __device__ __forceinline__ void ph_async_bfs(const Params &p, AsyncShared &sh, i
   const AsyncOwn own = async_own(p.n);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     c->aidle[1] = 0;  // the push phase's words
-    c->astop = 0;
+    c->adeadline = 0;
     c->aunsettled = 0;
     c->aact = 0;
     c->adepth = 0;
@@ -371,16 +374,16 @@ __device__ __forceinline__ void ph_async_finalize(const Params &p, bool write_si
 // of more than 8 arcs is discharged by its whole warp.  As in the rounds, a
 // vertex is only ever discharged by one thread or warp at a time, only its own
 // discharges lower its residuals and excess, and heights only rise, so the
-// races are those of the rounds.  Ends when no vertex is active, or after
-// budget_ns (set by the grid's first thread): the next relabel then gives exact
-// distances again.
+// races are those of the rounds.  Ends when no vertex is active, or budget_ns
+// after its start (a deadline that the grid's first thread sets and every block
+// keeps): the next relabel then gives exact distances again.
 // One window per warp, every narrow vertex of it with at most D arcs: heads,
 // partners and the label (only the owner changes it) sit in registers, and a
 // discharge is one round of loads, up to `cycles` pushes and relabels on what
 // they gave, and the atomics.
 template <int D>
-__device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh, const AsyncOwn &own, bool live, bool lead,
-                                               unsigned long long t0, unsigned long long budget_ns, LStats &ls) {
+__device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh, const AsyncOwn &own, bool live,
+                                               LStats &ls) {
   Ctrl *c = p.ctrl;
   const int lane = threadIdx.x & 31, v = own.first + lane;
   int beg = 0, deg = 0, h = p.n;
@@ -402,10 +405,9 @@ __device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh,
   for (int poll = 0;; poll++) {
     const long long ex = live ? ld_rlx(p.excess + v) : 0;
     const bool act = ex > 0 && h < p.n;
-    if (lead && (poll & 7) == 0 && globaltimer() - t0 > budget_ns) atomicExch(&c->astop, 1);
-    async_look(sh, poll, &c->astop, &c->err);
+    async_look(p, sh, poll, true);
     if (!__any_sync(0xffffffffu, act)) {
-      if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) break;
+      if (async_quiet(sh, st, own.count > 0, &c->aidle[1])) break;
       continue;
     }
     async_wake(sh, st, &c->aidle[1]);
@@ -468,7 +470,6 @@ __device__ __forceinline__ void async_push_one(const Params &p, AsyncShared &sh,
 
 // The same for a warp of several windows.
 __device__ __forceinline__ void async_push_loop(const Params &p, AsyncShared &sh, const AsyncOwn &own, unsigned live,
-                                                bool lead, unsigned long long t0, unsigned long long budget_ns,
                                                 LStats &ls) {
   Ctrl *c = p.ctrl;
   const int lane = threadIdx.x & 31;
@@ -514,11 +515,10 @@ __device__ __forceinline__ void async_push_loop(const Params &p, AsyncShared &sh
       }
       any = __any_sync(0xffffffffu, any);
     }
-    if (lead && (poll & 7) == 0 && globaltimer() - t0 > budget_ns) atomicExch(&c->astop, 1);
-    async_look(sh, poll, &c->astop, &c->err);
+    async_look(p, sh, poll, true);
     if (any) {
       if (async_stopped(sh)) break;
-    } else if (async_quiet(sh, st, own.count > 0, poll, &c->aidle[1], &c->astop, &c->err)) {
+    } else if (async_quiet(sh, st, own.count > 0, &c->aidle[1])) {
       break;
     }
   }
@@ -529,10 +529,8 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
   Ctrl *c = p.ctrl;
   const AsyncOwn own = async_own(p.n);
   const int lane = threadIdx.x & 31;
-  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-  unsigned long long t0 = 0;
-  if (lead) {
-    t0 = globaltimer();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *(volatile unsigned long long *)&c->adeadline = globaltimer() + budget_ns;
     c->pos_count = 0;
     c->unexplored = 0;
   }
@@ -549,11 +547,11 @@ __device__ __forceinline__ void ph_async_push(const Params &p, AsyncShared &sh, 
     const int v = own.first + lane;
     const int deg = live & 1 ? deg_of(p, v) : 0;
     if (__any_sync(0xffffffffu, deg > 4 && deg <= kSmallMax))
-      async_push_one<kSmallMax>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
+      async_push_one<kSmallMax>(p, sh, own, live & 1, ls);
     else
-      async_push_one<4>(p, sh, own, live & 1, lead, t0, budget_ns, ls);
+      async_push_one<4>(p, sh, own, live & 1, ls);
   } else {
-    async_push_loop(p, sh, own, live, lead, t0, budget_ns, ls);
+    async_push_loop(p, sh, own, live, ls);
   }
   async_end(sh, &c->aidle[1]);
   sink_flush(p, ls);

@@ -77,11 +77,12 @@ struct Ctrl {
   int berr, berr_info;          // error bits of a batch's lookup, and the update
   int nreopen;                  // updates queued for saturation: source arcs, reopened arcs
   int nrepair;                  // updates queued for the over-capacity repair
-  // barrier-free phases (dmf_async.cuh): blocks idle in the relabel [0] and in
-  // the push phase [1], the push phase's stop word, vertices whose label is not
-  // settled, active vertices and greatest distance of the last relabel
+  // barrier-free phases (dmf_async.cuh): when the push phase ends (0: not set
+  // yet), blocks idle in the relabel [0] and in the push phase [1], vertices whose
+  // label is not settled, active vertices and greatest distance of the last
+  // relabel
+  unsigned long long adeadline;
   int aidle[2];
-  int astop;
   int aunsettled;
   int aact;
   int adepth;

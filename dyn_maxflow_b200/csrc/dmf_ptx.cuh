@@ -35,6 +35,9 @@ __device__ __forceinline__ long long ld_rlx(const long long *p) {
   asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned long long ld_rlx(const unsigned long long *p) {
+  return (unsigned long long)ld_rlx((const long long *)p);
+}
 __device__ __forceinline__ unsigned long long globaltimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

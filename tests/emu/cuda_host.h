@@ -241,6 +241,7 @@ inline unsigned atom_add_acqrel_u32(unsigned *p, unsigned x) { return __atomic_f
 inline void st_release_sys_u32(unsigned *p, unsigned x) { __atomic_store_n(p, x, __ATOMIC_RELEASE); }
 inline int ld_rlx(const int *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 inline long long ld_rlx(const long long *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
+inline unsigned long long ld_rlx(const unsigned long long *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 inline unsigned long long globaltimer() {
   if (emu::fake_tick) return emu::fake_now->fetch_add(emu::fake_tick);
   return (unsigned long long)std::chrono::steady_clock::now().time_since_epoch().count();

@@ -58,3 +58,10 @@ def test_deep_solve_stays_together(kernel_main, oracle, tmp_path, n, width, bloc
     got, want = solve(kernel_main, oracle, tmp_path, n, width, blocks, warps, 0)
     assert [x[0] for x in got] == want
     assert got[0][1] > 0  # the greatest distance of a barrier-free relabel: there was one
+
+
+# a push phase past its time limit, with one window a warp and with several: a block that other blocks wait for, but
+# the first one does not, stops as well, long before the labels of its two vertices have climbed to n
+@pytest.mark.parametrize("blocks,n", [(2, 64), (2, 256), (3, 96), (3, 384)])
+def test_every_block_keeps_the_time_limit(kernel_main, blocks, n):
+    assert run(kernel_main, "push", blocks, n)[0][0] < n
