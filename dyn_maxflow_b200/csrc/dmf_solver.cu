@@ -9,6 +9,7 @@
 #include <climits>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <thread>
 #include <vector>
 
@@ -197,10 +198,15 @@ struct dmf_solver {
   HostResult *h_res = nullptr;  // pinned: what the last launch left
   unsigned seq = 0;             // number of the last launch
   bool direct = false;          // the staged batch is read from pinned host memory
-  bool ms_pending = false;      // st.last_ms is not read from the events yet
+  // Times of the calls: a call records the pair of events that the last call to
+  // end did not use, so that call's pair stays readable until another one ends
+  // (staging a batch records a start, and no solve may follow).
+  cudaEvent_t ev0[2] = {nullptr, nullptr}, ev1[2] = {nullptr, nullptr};
+  int ev_last = 0;
+  bool ms_pending = false;  // st.last_ms is not read from pair ev_last yet
+  std::mutex ms_mu;         // resolve_ms: several threads may ask for the statistics
   unsigned long long *trace = nullptr;  // device timeline (opts.flags & DMF_FLAG_TRACE)
   int trace_cap = 0;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   unsigned round_base = 1;
   int epoch = 0;
   bool solved = false, side_valid = false;
@@ -253,11 +259,11 @@ void free_all(dmf_solver *sv) {
   sv->h_inst_active = nullptr;
   if (sv->own_stream) cudaStreamDestroy(sv->own_stream);
   sv->own_stream = nullptr;
-  if (sv->ev0) cudaEventDestroy(sv->ev0);
-  if (sv->ev1) cudaEventDestroy(sv->ev1);
+  for (cudaEvent_t e : {sv->ev0[0], sv->ev0[1], sv->ev1[0], sv->ev1[1]})
+    if (e) cudaEventDestroy(e);
   sv->h_ubuf = nullptr;
   sv->h_res = nullptr;
-  sv->ev0 = sv->ev1 = nullptr;
+  sv->ev0[0] = sv->ev0[1] = sv->ev1[0] = sv->ev1[1] = nullptr;
 }
 
 constexpr int kTinyVertices = kBlock, kTinyArcs = 8 * kBlock;
@@ -448,6 +454,10 @@ int launch(dmf_solver *sv, int mode, int k, const int *d_src, const int *d_dst, 
   return DMF_OK;
 }
 
+// The events of the call that is under way.
+cudaEvent_t start_event(const dmf_solver *sv) { return sv->ev0[sv->ev_last ^ 1]; }
+cudaEvent_t end_event(const dmf_solver *sv) { return sv->ev1[sv->ev_last ^ 1]; }
+
 // Waits until the launch's result is in pinned memory: polls its number there
 // (a few us less than an event wait), and the event now and then, so that a
 // launch that failed ends the wait too.
@@ -455,7 +465,7 @@ int wait_result(dmf_solver *sv) {
   for (unsigned spin = 1;; spin++) {
     if (__atomic_load_n(&sv->h_res->seq, __ATOMIC_ACQUIRE) == sv->seq) return DMF_OK;
     if (spin % 4096 == 0) {
-      const cudaError_t q = cudaEventQuery(sv->ev1);
+      const cudaError_t q = cudaEventQuery(end_event(sv));
       if (q == cudaSuccess) {
         if (__atomic_load_n(&sv->h_res->seq, __ATOMIC_ACQUIRE) == sv->seq) return DMF_OK;
         return fail(DMF_ERR_CUDA, "the solve kernel left no result");
@@ -466,22 +476,31 @@ int wait_result(dmf_solver *sv) {
   }
 }
 
-// Device time of the last call, read from its events when somebody asks.
+// Device time of the last call, read from its events when somebody asks (waiting
+// for the end event in every call costs a few us).  Asking changes nothing for
+// the caller: any thread may, events need no current device, and the two calls
+// are made in relaxed capture mode, as the caller may be capturing a stream of
+// its own (these events are on no captured stream).
 void resolve_ms(const dmf_solver *csv) {
   dmf_solver *sv = const_cast<dmf_solver *>(csv);
+  std::lock_guard<std::mutex> lock(sv->ms_mu);
   if (!sv->ms_pending) return;
   sv->ms_pending = false;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   float ms = 0;
-  if (cudaSetDevice(sv->dev) == cudaSuccess && cudaEventSynchronize(sv->ev1) == cudaSuccess &&
-      cudaEventElapsedTime(&ms, sv->ev0, sv->ev1) == cudaSuccess)
+  if (cudaEventSynchronize(sv->ev1[sv->ev_last]) == cudaSuccess &&
+      cudaEventElapsedTime(&ms, sv->ev0[sv->ev_last], sv->ev1[sv->ev_last]) == cudaSuccess)
     sv->st.last_ms = ms;
+  cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 // Waits for the launch sequence, records timing and maps device errors.
 int finish(dmf_solver *sv, int64_t *flow, bool need_cut_valid) {
-  CK(cudaEventRecord(sv->ev1, sv->stream), "event record");
+  CK(cudaEventRecord(end_event(sv), sv->stream), "event record");
   if (int st = wait_result(sv)) return st;
   const Ctrl &c = sv->h_res->c;
+  sv->ev_last ^= 1;
   sv->ms_pending = true;
   sv->st.outer_iters = (int64_t)c.st_outer;
   sv->st.bfs_levels = (int64_t)c.st_levels;
@@ -545,7 +564,7 @@ int finish(dmf_solver *sv, int64_t *flow, bool need_cut_valid) {
 
 int run_mode(dmf_solver *sv, int mode, int k, const int *d_src, const int *d_dst, const int *d_w, int64_t *flow,
              bool started) {
-  if (!started) CK(cudaEventRecord(sv->ev0, sv->stream), "event record");
+  if (!started) CK(cudaEventRecord(start_event(sv), sv->stream), "event record");
   int st = launch(sv, mode, k, d_src, d_dst, d_w);
   if (st) return st;
   return finish(sv, flow, sv->opts.variant == DMF_VARIANT_PP || mode == MODE_CUT);
@@ -631,7 +650,7 @@ int stage_batch(dmf_solver *sv, int32_t k, const int32_t *src, const int32_t *ds
     }
     if (err != cudaSuccess) return cuda_fail(err, "H2D batch");
   }
-  CK(cudaEventRecord(sv->ev0, sv->stream), "event record");
+  CK(cudaEventRecord(start_event(sv), sv->stream), "event record");
   return DMF_OK;
 }
 
@@ -1019,8 +1038,8 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
   if (e == cudaSuccess) e = cudaHostAlloc((void **)&sv->h_res, sizeof(HostResult), cudaHostAllocMapped);
   if (e == cudaSuccess) std::memset((void *)sv->h_res, 0, sizeof(HostResult));
   if (e == cudaSuccess) e = cudaMemsetAsync(sv->ctrl, 0, sizeof(Ctrl), S);
-  if (e == cudaSuccess) e = cudaEventCreate(&sv->ev0);
-  if (e == cudaSuccess) e = cudaEventCreate(&sv->ev1);
+  for (cudaEvent_t *ev : {&sv->ev0[0], &sv->ev0[1], &sv->ev1[0], &sv->ev1[1]})
+    if (e == cudaSuccess) e = cudaEventCreate(ev);
   if (e == cudaSuccess) e = cudaStreamSynchronize(S);
   if (e != cudaSuccess) return cuda_fail(e, "solver upload");
   // Staging up front: on the device for an eighth of the arcs, up to 2^18 updates,
@@ -1277,10 +1296,10 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
       }
       if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     }
-    if (e == cudaSuccess) e = cudaEventRecord(sv->ev0, S);
+    if (e == cudaSuccess) e = cudaEventRecord(start_event(sv), S);
     if (e == cudaSuccess) e = use_graph ? cudaGraphLaunch(exec, S) : enqueue_steps();
-    if (e == cudaSuccess) e = cudaEventRecord(sv->ev1, S);
-    if (e == cudaSuccess) e = cudaEventSynchronize(sv->ev1);
+    if (e == cudaSuccess) e = cudaEventRecord(end_event(sv), S);
+    if (e == cudaSuccess) e = cudaEventSynchronize(end_event(sv));
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
@@ -1289,7 +1308,7 @@ int dmf_multi_run_batches(dmf_solver *sv, int32_t steps, const int64_t *ofs, con
       return cuda_fail(e, use_graph ? "graph-captured batch loop" : "batch loop");
     }
     float t_ms = 0;
-    cudaEventElapsedTime(&t_ms, sv->ev0, sv->ev1);
+    cudaEventElapsedTime(&t_ms, start_event(sv), end_event(sv));
     if (ms) *ms = t_ms;
     int rc = DMF_OK;
     unsigned outer = 0;
