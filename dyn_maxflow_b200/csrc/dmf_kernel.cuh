@@ -2311,7 +2311,10 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     if (!p.caps_bounded && !sc->berr) {
       kind = TR_APPLY;
       ph_claim_apply(p, dyn);
-      if (!next()) return;
+      if (!next()) {
+        ph_unclaim(p, dyn);
+        return;
+      }
     }
     if (sc->berr || sc->dup_at) {  // every claim is done: undo them, reject the batch
       if (p.caps_bounded || !sc->berr) ph_unclaim(p, dyn);

@@ -146,6 +146,7 @@ inline T reduce(unsigned mask, T x, F f) {
   return r;
 }
 
+inline int skip_barrier = 0;  // the grid barrier (1: the first) that the last block never arrives at
 inline unsigned long long fake_tick = 0;  // 0: real time; else ns that every look at the clock takes
 inline std::atomic<unsigned long long> *fake_now = nullptr;
 
@@ -236,7 +237,11 @@ inline void __threadfence_system() { __atomic_thread_fence(__ATOMIC_SEQ_CST); }
 #define DMF_PTX_CUH
 namespace dmfd {
 inline unsigned ld_acquire_u32(const unsigned *p) { sched_yield(); return __atomic_load_n(p, __ATOMIC_ACQUIRE); }
-inline unsigned atom_add_release_u32(unsigned *p, unsigned x) { return __atomic_fetch_add(p, x, __ATOMIC_SEQ_CST); }
+inline unsigned atom_add_release_u32(unsigned *p, unsigned x) {  // only grid barriers use it
+  static int count = 0;
+  if (blockIdx.x == gridDim.x - 1 && ++count == emu::skip_barrier) return __atomic_load_n(p, __ATOMIC_SEQ_CST);
+  return __atomic_fetch_add(p, x, __ATOMIC_SEQ_CST);
+}
 inline unsigned atom_add_acqrel_u32(unsigned *p, unsigned x) { return __atomic_fetch_add(p, x, __ATOMIC_SEQ_CST); }
 inline void st_release_sys_u32(unsigned *p, unsigned x) { __atomic_store_n(p, x, __ATOMIC_RELEASE); }
 inline int ld_rlx(const int *p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }

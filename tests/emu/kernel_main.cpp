@@ -1,5 +1,7 @@
 // kernel_main.cpp -- the solve kernel on host threads (cuda_host.h).
 //   kernel_main solve FILE BLOCKS THREADS VARIANT   flow of a solve from scratch, then of the file's batch
+//   kernel_main timeout FILE BLOCKS THREADS BARRIER  the batch with a grid barrier that a block never arrives at:
+//                                                   the error word, and what differs in capacities and residuals
 //   kernel_main push BLOCKS N                       a push phase past its time limit: does every block stop?
 // FILE: int32 n, m, s, t, k, then index[n+1], adj[m], cap[m], par[m], src[k], dst[k], w[k].
 #include "cuda_host.h"
@@ -101,13 +103,18 @@ struct Device {
   }
 };
 
-int solve(char **a) {
-  FILE *f = std::fopen(a[0], "rb");
+Device load(const char *path) {
+  FILE *f = std::fopen(path, "rb");
   int h[5];
-  if (!f || fread(h, 4, 5, f) != 5) return 2;
+  if (!f || fread(h, 4, 5, f) != 5) std::abort();
   Device d(h[0], h[1], h[2], h[3], h[4]);
   d.graph(f);
   std::fclose(f);
+  return d;
+}
+
+int solve(char **a) {
+  Device d = load(a[0]);
   const int blocks = std::atoi(a[1]), threads = std::atoi(a[2]);
   d.p.variant = std::atoi(a[3]);
   d.p.need_cut = d.p.variant == DMF_VARIANT_PP;
@@ -116,6 +123,22 @@ int solve(char **a) {
     if (err) return err < 0 ? 3 : 5;
     std::printf("%lld %d\n", d.res->c.flow, d.res->c.adepth);
   }
+  return 0;
+}
+
+int timeout(char **a) {
+  Device d = load(a[0]);
+  const int blocks = std::atoi(a[1]), threads = std::atoi(a[2]);
+  if (d.run(MODE_STATIC, blocks, threads)) return 3;
+  std::vector<unsigned> cap(d.p.m);
+  for (int e = 0; e < d.p.m; e++) cap[e] = (unsigned)d.p.capx[e];
+  const std::vector<int> res(d.p.res, d.p.res + d.p.m);
+  emu::skip_barrier = std::atoi(a[3]);
+  d.p.barrier_ns = kSecond / 5;
+  const int err = d.run(MODE_DYNAMIC, blocks, threads);
+  int diff = 0;
+  for (int e = 0; e < d.p.m; e++) diff += cap[e] != (unsigned)d.p.capx[e] || res[e] != d.p.res[e];
+  std::printf("%d %d\n", err, diff);
   return 0;
 }
 
@@ -149,6 +172,7 @@ int push(char **a) {
 
 int main(int argc, char **argv) {
   if (argc == 6 && !std::strcmp(argv[1], "solve")) return solve(argv + 2);
+  if (argc == 6 && !std::strcmp(argv[1], "timeout")) return timeout(argv + 2);
   if (argc == 4 && !std::strcmp(argv[1], "push")) return push(argv + 2);
   return 2;
 }

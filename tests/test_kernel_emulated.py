@@ -36,26 +36,29 @@ def ladder(oracle, n, width, seed):
     return oracle.build_csr(a, b, rng.integers(1, 50, len(a)))
 
 
-def solve(kernel_main, oracle, tmp_path, n, width, blocks, warps, variant):
+def write(oracle, path, n, width, big=0):
+    """A ladder and a batch as kernel_main reads them; the flows before and after the batch."""
     got_n, m, off, adj, cap, par = ladder(oracle, n, width, n)
     assert got_n == n
+    if big:
+        cap[0] = big
     rng = np.random.default_rng(n + 1)
     arcs = rng.permutation(m)[:m // 10]
     src, dst = np.searchsorted(off, arcs, side="right") - 1, adj[arcs]
     to = rng.integers(0, 60, len(arcs))
-    path = str(tmp_path / "graph")
     np.concatenate([[n, m, n - 2, n - 1, len(arcs)], off, adj, cap, par, src, dst, to]).astype(np.int32).tofile(path)
     new = cap.copy()
     new[arcs] = to
-    want = [oracle.dinic(n, off, adj, c, par, n - 2, n - 1) for c in (cap, new)]
-    return run(kernel_main, "solve", path, blocks, 32 * warps, variant), want
+    return [oracle.dinic(n, off, adj, c, par, n - 2, n - 1) for c in (cap, new)]
 
 
 # deep graphs: every warp one window of 32 vertices, some none, some more than others, the most a warp can own
 @pytest.mark.parametrize("n,width,blocks,warps", [(64, 1, 1, 2), (64, 2, 2, 2), (30, 1, 1, 2), (96, 1, 1, 2),
                                                   (97, 2, 1, 2), (160, 3, 2, 2), (200, 2, 1, 4), (256, 4, 1, 2)])
 def test_deep_solve_stays_together(kernel_main, oracle, tmp_path, n, width, blocks, warps):
-    got, want = solve(kernel_main, oracle, tmp_path, n, width, blocks, warps, 0)
+    path = str(tmp_path / "graph")
+    want = write(oracle, path, n, width)
+    got = run(kernel_main, "solve", path, blocks, 32 * warps, 0)
     assert [x[0] for x in got] == want
     assert got[0][1] > 0  # the greatest distance of a barrier-free relabel: there was one
 
@@ -65,3 +68,13 @@ def test_deep_solve_stays_together(kernel_main, oracle, tmp_path, n, width, bloc
 @pytest.mark.parametrize("blocks,n", [(2, 64), (2, 256), (3, 96), (3, 384)])
 def test_every_block_keeps_the_time_limit(kernel_main, blocks, n):
     assert run(kernel_main, "push", blocks, n)[0][0] < n
+
+
+# a batch whose barrier wait runs out leaves capacities and residuals as they were: the claim is in the first phase, or
+# (one capacity above 2^30 - 1) in a second one after a barrier
+@pytest.mark.parametrize("big,barrier", [(0, 1), (2**30 + 5, 1), (2**30 + 5, 2)])
+def test_timed_out_batch_takes_its_claims_back(kernel_main, oracle, tmp_path, big, barrier):
+    path = str(tmp_path / "graph")
+    write(oracle, path, 200, 20, big)
+    err_timeout = 1
+    assert run(kernel_main, "timeout", path, 2, 64, barrier) == [[err_timeout, 0]]
