@@ -302,8 +302,9 @@ int configure(dmf_solver *sv) {
   if (sv->opts.grid_blocks > 0) sv->grid = std::min(sv->grid, sv->opts.grid_blocks);
   // A graph that one block's threads cover has no use for a second block, and a
   // grid of one needs no grid barrier (420 arcs: 1.22 times as fast by the host
-  // clock, with the plain sweeps; 0.5 M arcs would lose: 90 us against 66).
-  if (sv->n <= kTinyVertices && sv->m <= kTinyArcs) sv->grid = 1;
+  // clock, with the plain sweeps; 0.5 M arcs would lose: 90 us against 66).  The
+  // barrier hook needs a second block, whose barrier it can let run out.
+  if (sv->n <= kTinyVertices && sv->m <= kTinyArcs && !(sv->opts.flags & DMF_FLAG_TEST_BARRIER_TIMEOUT)) sv->grid = 1;
   if (sv->opts.small_deg > 0) sv->small_deg = sv->opts.small_deg;
   else if (sv->opts.small_deg < 0) sv->small_deg = 0;  // no thread tier
   sv->block = kBlock;

@@ -84,3 +84,17 @@ def test_barrier_timeout_returns_instead_of_hanging(dmf, oracle, variant):
         assert sv.static_maxflow() == want
         assert sv.apply_updates(*batches[0]) == want1
         _certified(oracle, g, sv, s, t, want1)
+
+
+def test_barrier_timeout_on_a_graph_of_one_block(dmf, oracle):
+    # a graph that a single block would solve without any grid barrier
+    g, s, t = dmf.gen_rmat(7, 8 << 7, seed=7, cap_lo=1, cap_hi=1000)
+    want = _exact(oracle, g, s, t)
+    with dmf.Solver(g, s, t, test_barrier_timeout=True) as sv:
+        with pytest.raises(dmf.DmfError) as ei:
+            sv.static_maxflow()
+        assert ei.value.status == DMF_ERR_TIMEOUT
+        sv.set_opts(flags=0)
+        assert sv.static_maxflow() == want
+        assert sv.stats()["grid_blocks"] == 1
+        _certified(oracle, g, sv, s, t, want)
