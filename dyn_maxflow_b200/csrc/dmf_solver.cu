@@ -1076,7 +1076,7 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
       if (cudaMemcpy(sv->role, ms->role.data(), ms->role.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
           cudaMemcpy(sv->inst, ms->inst.data(), 4 * ms->inst.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
           cudaHostAlloc((void **)&sv->h_inst_flow, 8 * (size_t)ms->count, cudaHostAllocMapped) != cudaSuccess ||
-          cudaMemset(sv->inst_flow, 0, 8 * (size_t)ms->count) != cudaSuccess)
+          cudaMemsetAsync(sv->inst_flow, 0, 8 * (size_t)ms->count, S) != cudaSuccess)
         return cuda_fail(cudaGetLastError(), "batched-instance upload");
     }
   }
