@@ -27,6 +27,15 @@ constexpr int kAsyncWin = 4;
 // takes to become visible, so that a wave crossing from one block to another
 // does not find every block idle.
 constexpr int kQuietPolls = 8;
+// A sink's row longer than this is relaxed by a level-synchronous level at the
+// start of every relabel, over the whole grid, before the barrier-free phase: one
+// warp takes it 128 arcs in about 0.8 us, the seeds with their frontier and the
+// level about 25 us for any length.  Segmentation graphs (every vertex of a grid
+// joined to s and t), static solve with the level / without / barriers throughout:
+// 1,024 arcs 0.96 / 0.98 / 1.9 ms, 2,304 arcs 0.65 / 0.75 / 1.5, 65,536 arcs 1.05 /
+// 6.6 / 3.4, 262,144 arcs 3.0 / 16 / 7.2.  Other long rows stay with one warp: a
+// hub of 100,000 arcs on a ladder, 43 ms against 220 with barriers throughout.
+constexpr int kWideSink = 2048;
 // Polls of a block's first warp in a phase at most (bounds the loop, whatever
 // the polls find; a phase is far shorter).
 constexpr int kMaxPolls = 1 << 20;
@@ -135,14 +144,34 @@ __device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool
 // Labels only fall and every fall is seen by its owner, so once no vertex has a
 // label below the one it last relaxed from (ph_async_settled, between two
 // barriers) the labels are the exact distances.
-// Relaxes the tails of a long row's residual in-arcs, by a whole warp.
+
+// Relaxes the tails of a long row's residual in-arcs, by a whole warp, kRelaxBatch
+// arcs a lane with their loads in flight together.  No other warp helps with the
+// row, so everything behind it waits (65,536 arcs: about 0.5 ms; one arc a lane at
+// a time about 2 ms; 8 were no faster than 4).
+constexpr int kRelaxBatch = 4;
+
 __device__ __forceinline__ void async_relax_row(const Params &p, int v, int h, LStats &ls) {
   const int b = __ldg(p.off + v), e = __ldg(p.off + v + 1);
-  for (int a = b + (int)(threadIdx.x & 31); a < e; a += 32) {
-    const int w = __ldg(p.adj + a);
-    ls.barcs++;
-    const int cur = __ldcg(p.height + w);
-    if (cur > h + 1 && cur != p.n && __ldcg(p.res + __ldg(p.par + a)) > 0) atomicMin(p.height + w, h + 1);
+  for (int a0 = b + (int)(threadIdx.x & 31); a0 < e; a0 += 32 * kRelaxBatch) {
+    int w[kRelaxBatch], r[kRelaxBatch];
+#pragma unroll
+    for (int k = 0; k < kRelaxBatch; k++) {
+      const int a = a0 + 32 * k;
+      w[k] = a < e ? __ldg(p.adj + a) : -1;
+      r[k] = a < e ? __ldg(p.par + a) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kRelaxBatch; k++) {
+      if (w[k] < 0) continue;
+      ls.barcs++;
+      const int cur = __ldcg(p.height + w[k]);
+      r[k] = __ldcg(p.res + r[k]);
+      if (cur <= h + 1 || cur == p.n) r[k] = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kRelaxBatch; k++)
+      if (w[k] >= 0 && r[k] > 0) atomicMin(p.height + w[k], h + 1);
   }
   __syncwarp();
 }

@@ -82,6 +82,7 @@ struct Params {
   int *lq, *lst;
   unsigned char *inl;
   int nact;                    // vertices of the instances this call works on
+  int sink_deg;                // arcs of the sink (the most that one has, in batched mode)
   int *pcur;                   // per vertex: where in its row its last pull found enough (long rows; may be null)
   int2 *fh[2], *wh[2], *ah;    // hub chunk queues
   const int2 *hch;             // every hub's chunks (bottom-up BFS, topology-driven rounds)
@@ -2352,6 +2353,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   // Deep graphs: once a relabel has gone kDeepLevels levels, it and the rest of
   // the solve use the barrier-free phases, where the grid can own every vertex.
   const bool deep_ok = p.adaptive && p.interval <= kDeepLevels && async_fits(p.n);
+  const bool wide_sink = p.sink_deg > kWideSink;
 
   // ---- local repair inside the kept dead set ------------------------------------
   // The first global relabel revives every vertex, unless the dead set of the
@@ -2479,7 +2481,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     }
     kind = TR_BFS_INIT;
     items = hubitems = 0;
-    if (deep) ph_deep_init(p);
+    if (deep && !wide_sink) ph_deep_init(p);
     else ph_bfs_init(p, slot_out(), it == 0 && revive, it == 0 && !revive, listed);
     if (!next()) return;
     if (lead) c->st_outer++;
@@ -2490,7 +2492,7 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     bool bu = false, full = true;
     int L = 0, reached = 0;
     for (;; L++) {
-      if (deep) break;
+      if (deep && !(wide_sink && L == 0)) break;
       const Slot *in = slot_in();
       const int F = in->q + in->hq;
       const long long m_f = in->arcs;

@@ -182,6 +182,7 @@ struct dmf_solver {
   int *srcs = nullptr;
   int *src_off = nullptr;  // prefix sums of the sources' degrees
   int nsrc = 1;
+  int sink_deg = 0;        // arcs of the sink with the most
   long long *inst_flow = nullptr;
   long long *h_inst_flow = nullptr;  // pinned
   std::vector<int> vbase;            // first vertex of each instance in the union
@@ -377,6 +378,7 @@ Params make_params(dmf_solver *sv, int mode, int k, const int *d_src, const int 
   p.lst = sv->lst;
   p.inl = sv->inl;
   p.nact = sv->n;
+  p.sink_deg = sv->sink_deg;
   if (sv->use_active) {
     p.nact = 0;
     for (int i = 0; i < sv->ninst; i++)
@@ -978,6 +980,8 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
       (st = dalloc(sv, &sv->qbuf, 6 * N)) || (st = dalloc(sv, &sv->dlab, N)) || (st = dalloc(sv, &sv->pcur, N)) || (st = dalloc(sv, &sv->lq, N)) ||
       (st = dalloc(sv, &sv->lst, 1)) || (st = dalloc(sv, &sv->inl, N)) || (st = dalloc(sv, &sv->ctrl, 1)))
     return st;
+  for (int v = 0; v < g->n; v++)
+    if (ms ? (ms->role[v] & 2) != 0 : v == t) sv->sink_deg = std::max(sv->sink_deg, g->off[v + 1] - g->off[v]);
   std::vector<int2> hub_chunks;
   std::vector<int> hub_base(g->n, -1);
   for (int v = 0; v < g->n; v++) {

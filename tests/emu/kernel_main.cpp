@@ -1,5 +1,7 @@
 // kernel_main.cpp -- the solve kernel on host threads (cuda_host.h).
-//   kernel_main solve FILE BLOCKS THREADS VARIANT   flow of a solve from scratch, then of the file's batch
+//   kernel_main solve FILE BLOCKS THREADS SINK_DEG  flow of a solve from scratch, then of the file's batch, each with
+//                                                   the number of barrier-free relabels and push phases it had
+//                                                   (SINK_DEG: the sink's degree the kernel is told, 0: the true one)
 //   kernel_main timeout FILE BLOCKS THREADS BARRIER  the batch with a grid barrier that a block never arrives at:
 //                                                   the error word, and what differs in capacities and residuals
 //   kernel_main push BLOCKS N                       a push phase past its time limit: does every block stop?
@@ -61,6 +63,14 @@ struct Device {
     p.round_base = p.relabel_base = 1;
     p.barrier_ns = 30 * kSecond;
     p.absent_block = -1;
+    p.trace_cap = 1 << 14;
+    p.trace = emu::global<unsigned long long>(4 * (size_t)p.trace_cap);
+  }
+
+  int phases(int kind) const {
+    int count = 0;
+    for (int i = 0; i < res->c.trace_len; i++) count += (int)(p.trace[4 * i] & 0xff) == kind;
+    return count;
   }
 
   const int *ints(FILE *f, size_t count) {
@@ -74,6 +84,7 @@ struct Device {
     p.adj = ints(f, p.m);
     const int *cap = ints(f, p.m);
     p.par = ints(f, p.m);
+    p.sink_deg = p.off[p.t + 1] - p.off[p.t];
     p.usrc = p.xsrc = ints(f, p.k);
     p.udst = p.xdst = ints(f, p.k);
     p.uw = p.xw = ints(f, p.k);
@@ -116,12 +127,11 @@ Device load(const char *path) {
 int solve(char **a) {
   Device d = load(a[0]);
   const int blocks = std::atoi(a[1]), threads = std::atoi(a[2]);
-  d.p.variant = std::atoi(a[3]);
-  d.p.need_cut = d.p.variant == DMF_VARIANT_PP;
+  if (std::atoi(a[3])) d.p.sink_deg = std::atoi(a[3]);
   for (int mode : {MODE_STATIC, MODE_DYNAMIC}) {
     const int err = d.run(mode, blocks, threads);
     if (err) return err < 0 ? 3 : 5;
-    std::printf("%lld %d\n", d.res->c.flow, d.res->c.adepth);
+    std::printf("%lld %d %d\n", d.res->c.flow, d.phases(TR_BFS_ASYNC), d.phases(TR_PUSH_ASYNC));
   }
   return 0;
 }

@@ -94,3 +94,24 @@ def test_masked_instances(dmf, oracle):
                 parts.append((np.full(len(b[0]), i), *b))
             got = ms.apply_updates_all(*(np.concatenate(x) for x in zip(*parts)))
             assert got.tolist() == [want(i) for i in range(4)]
+
+
+# a sink joined to every vertex of a grid: at, just above and far above the arcs from which its row gets a level of its
+# own at the start of a barrier-free relabel
+@pytest.mark.parametrize("variant", ("data", "pp"))
+@pytest.mark.parametrize("side", (45, 46, 150))
+def test_wide_sink(dmf, oracle, variant, side):
+    rng = np.random.default_rng(side)
+    v = np.arange(side * side).reshape(side, side)
+    right, down = v[:, :-1].ravel(), v[:-1].ravel()
+    a = np.concatenate([right, right + 1, down, down + side, np.full(side, v.size), v.ravel()])
+    b = np.concatenate([right + 1, right, down + side, down, v[0], np.full(v.size, v.size + 1)])
+    w = np.concatenate([rng.integers(20, 60, len(a) - side - v.size), np.full(side, 500), rng.integers(0, 4, v.size)])
+    g, s, t = dmf.Graph.from_edges(a, b, w), v.size, v.size + 1
+    index = g.arrays()[0]
+    assert index[t + 1] - index[t] == v.size
+    batches = dmf.gen_batches(g, 3, frac=0.05, p_inc=0.5, p_dec=0.4, p_ins=0.0, delta_hi=30, seed=side)
+    with dmf.Solver(g, s, t, variant=variant, trace=True) as sv:
+        assert sv.static_maxflow() > 0
+        assert "bfs_async" in [x[0] for x in sv.trace()]
+        solve_and_check(dmf, oracle, g, s, t, sv, batches)

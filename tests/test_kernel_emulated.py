@@ -26,19 +26,26 @@ def run(*args):
     return [[int(x) for x in line.split()] for line in r.stdout.splitlines()]
 
 
-def ladder(oracle, n, width, seed):
-    """Columns of `width` vertices, neighbours both ways, s before the first column and t after the last."""
+def ladder(oracle, n, width, seed, hubs=0):
+    """Columns of `width` vertices, neighbours both ways, s before the first column and t after the last; `hubs` more
+    vertices get flow from s and have an arc to every vertex of the columns (long rows, but no way in)."""
     rng = np.random.default_rng(seed)
-    u = np.arange(n - 2)
-    step, up = u[u + width < n - 2], u[(u + 1 < n - 2) & ((u + 1) % width != 0)]
-    a = np.concatenate([step, step + width, up, up + 1, np.full(width, n - 2), u[-width:]])
-    b = np.concatenate([step + width, step, up + 1, up, u[:width], np.full(width, n - 1)])
-    return oracle.build_csr(a, b, rng.integers(1, 50, len(a)))
+    inner, s, t = n - 2 - hubs, n - 2, n - 1
+    u = np.arange(inner)
+    step, up = u[u + width < inner], u[(u + 1 < inner) & ((u + 1) % width != 0)]
+    a = np.concatenate([step, step + width, up, up + 1, np.full(width, s), u[-width:]])
+    b = np.concatenate([step + width, step, up + 1, up, u[:width], np.full(width, t)])
+    w = rng.integers(1, 50, len(a))
+    for h in range(inner, s):
+        a = np.concatenate([a, [s], np.full(inner, h)])
+        b = np.concatenate([b, [h], u])
+        w = np.concatenate([w, [inner], np.ones(inner, np.int64)])
+    return oracle.build_csr(a, b, w)
 
 
-def write(oracle, path, n, width, big=0):
+def write(oracle, path, n, width, big=0, hubs=0):
     """A ladder and a batch as kernel_main reads them; the flows before and after the batch."""
-    got_n, m, off, adj, cap, par = ladder(oracle, n, width, n)
+    got_n, m, off, adj, cap, par = ladder(oracle, n, width, n, hubs)
     assert got_n == n
     if big:
         cap[0] = big
@@ -60,7 +67,7 @@ def test_deep_solve_stays_together(kernel_main, oracle, tmp_path, n, width, bloc
     want = write(oracle, path, n, width)
     got = run(kernel_main, "solve", path, blocks, 32 * warps, 0)
     assert [x[0] for x in got] == want
-    assert got[0][1] > 0  # the greatest distance of a barrier-free relabel: there was one
+    assert got[0][1] > 0  # it had barrier-free relabels
 
 
 # a push phase past its time limit, with one window a warp and with several: a block that other blocks wait for, but
@@ -68,6 +75,25 @@ def test_deep_solve_stays_together(kernel_main, oracle, tmp_path, n, width, bloc
 @pytest.mark.parametrize("blocks,n", [(2, 64), (2, 256), (3, 96), (3, 384)])
 def test_every_block_keeps_the_time_limit(kernel_main, blocks, n):
     assert run(kernel_main, "push", blocks, n)[0][0] < n
+
+
+# rows of 9 arcs and more go to a whole warp: below, at and above the arcs it takes at a time, and several times that
+@pytest.mark.parametrize("n", [36, 64, 127, 130, 131, 290, 500])
+def test_deep_solve_with_long_rows(kernel_main, oracle, tmp_path, n):
+    path = str(tmp_path / "graph")
+    want = write(oracle, path, n, 1 if n < 64 else 3, hubs=2)
+    got = run(kernel_main, "solve", path, 1, 128, 0)
+    assert [x[0] for x in got] == want
+    assert got[0][1] > 0
+
+
+# the sink's row by a level of its own before every barrier-free relabel, as for sinks of more than 2,048 arcs
+@pytest.mark.parametrize("n,width,hubs", [(64, 1, 0), (97, 2, 0), (130, 3, 2), (256, 40, 1)])
+def test_deep_solve_with_a_wide_sink(kernel_main, oracle, tmp_path, n, width, hubs):
+    path = str(tmp_path / "graph")
+    want = write(oracle, path, n, width, hubs=hubs)
+    assert [x[0] for x in run(kernel_main, "solve", path, 1, 128, 4097)] == want
+    assert [x[0] for x in run(kernel_main, "solve", path, 2, 128, 4097)] == want
 
 
 # a batch whose barrier wait runs out leaves capacities and residuals as they were: the claim is in the first phase, or
