@@ -194,7 +194,7 @@ __device__ __forceinline__ void set_batch_err(Ctrl *c, int bit, int info) {
 }
 
 // A dead vertex whose excess a batch lowers joins the candidate list once
-// (stamp = round_base, a value no push round of this call uses).  The pull
+// (stamp = round_base, a value no pull round of this call uses).  The pull
 // rounds later append the dead vertices they take below zero, so after them
 // the list holds every dead vertex that can hold a deficit (dead vertices end
 // every solve with excess >= 0).  The list has n + 1 entries; a count past
@@ -1540,8 +1540,7 @@ constexpr int kSmallMax = 8;
 // residuals and head heights of all arcs are loaded together, the pushes are
 // decided in registers (excess spread over the admissible arcs in arc order),
 // and every atomic of the cycle is in flight before any result is used; the
-// heads that became active are deduplicated by their stamps together and
-// appended with one reservation.  A head height may be one load old when it is
+// heads that a push made active (see enqueue) are appended with one reservation.  A head height may be one load old when it is
 // used (a concurrent relabel only raises it), which can leave a label above
 // the exact distance for a while; labels only steer the pushes -- dead
 // vertices and termination are decided by the exact BFS of each relabel.
@@ -1768,11 +1767,9 @@ struct RoundIn {
   int nh;
 };
 
-// dph: a round of the local repair inside the dead set (always worklist-driven:
-// a topology sweep would discharge live vertices too).
-__device__ __forceinline__ RoundIn round_inputs(const Params &p, const Ctrl *c, int r, bool dph) {
+__device__ __forceinline__ RoundIn round_inputs(const Params &p, const Ctrl *c, int r) {
   RoundIn in;
-  if (p.variant == DMF_VARIANT_TOPO && !dph) {
+  if (p.variant == DMF_VARIANT_TOPO) {
     in.nlist = nullptr;
     in.nn = p.n;
     in.hlist = p.hch;
@@ -1795,10 +1792,10 @@ __device__ __forceinline__ RoundIn round_inputs(const Params &p, const Ctrl *c, 
 // chunk sums its admissible residual, adds its minimum non-admissible head
 // height to the hub's, and pushes its share of the hub's excess.
 template <int TILE>
-__device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int r, unsigned gepoch, LStats &ls, bool dph) {
+__device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int r, unsigned gepoch, LStats &ls) {
   Ctrl *c = p.ctrl;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool topo = p.variant == DMF_VARIANT_TOPO && !dph;
+  const bool topo = p.variant == DMF_VARIANT_TOPO;
   if (gt == 0) {
     if (r == 0) {  // read during the BFS just finished; cleared for the next one
       c->pos_count = 0;
@@ -1929,9 +1926,9 @@ __device__ __forceinline__ void ph_push1(const Params &p, const RoundIn &in, int
 // its excess; when all of the hub's admissible residual was pushed and excess is
 // left, the hub is relabelled to 1 + the minimum non-admissible height; a hub
 // with excess left is queued for the next round.  The hub's totals are reset.
-__device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int r, LStats &ls, bool dph) {
+__device__ __forceinline__ void ph_push3(const Params &p, const RoundIn &in, int r, LStats &ls) {
   const int nt = gridDim.x * blockDim.x;
-  const bool topo = p.variant == DMF_VARIANT_TOPO && !dph;
+  const bool topo = p.variant == DMF_VARIANT_TOPO;
   int seen = 0;
   for (int i = spread_thread(); i < in.nh; i += nt) {
     const int2 it = __ldcg(in.hlist + i);
@@ -2352,6 +2349,11 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
   unsigned round_id = p.round_base;
   // Deep graphs: once a relabel has gone kDeepLevels levels, it and the rest of
   // the solve use the barrier-free phases, where the grid can own every vertex.
+  // Their push phase has no rounds, so they are left to solves that do not ask
+  // for a number of them: FIXED_INTERVAL promises exactly relabel_interval rounds
+  // a relabel, a relabel_interval above kDeepLevels more rounds than the levels
+  // that lead here, and the allocation-free solve runs a fixed schedule.  Those
+  // keep a barrier per level and round (256 x 256 grid: 150 ms against 16).
   const bool deep_ok = p.adaptive && p.interval <= kDeepLevels && async_fits(p.n);
   const bool wide_sink = p.sink_deg > kWideSink;
 
@@ -2558,22 +2560,18 @@ __device__ __forceinline__ void run(const Params &p, LStats &ls, Ctrl *sc, Async
     // worklist empties)
     const int rounds = (p.interval > L || !p.adaptive) ? p.interval : L;
     for (int r = 0; r < rounds; r++) {
-      round_id++;
-      const RoundIn in = round_inputs(p, sc, r, false);
+      const RoundIn in = round_inputs(p, sc, r);
       kind = TR_PUSH;
       items = in.nn;
       hubitems = in.nh;
-      ph_push1<TILE>(p, in, r, p.relabel_base + it, ls, false);
+      ph_push1<TILE>(p, in, r, p.relabel_base + it, ls);
       if (!next()) return;
       if (in.nh > 0) {
         kind = TR_PUSH_HUB_FINISH;
-        ph_push3(p, in, r, ls, false);
+        ph_push3(p, in, r, ls);
         if (!next()) return;
       }
-      if (lead) {
-        c->st_rounds++;
-        c->rounds_used = round_id - p.round_base;
-      }
+      if (lead) c->st_rounds++;
       const int W = topo ? sc->seen[r % 3] : sc->wtail[r % 3] + sc->whtail[r % 3];
       if (W == 0) break;
     }

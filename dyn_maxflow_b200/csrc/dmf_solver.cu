@@ -424,8 +424,6 @@ Params make_params(dmf_solver *sv, int mode, int k, const int *d_src, const int 
   p.ctrl = sv->ctrl;
   p.mode = mode;
   p.variant = sv->opts.variant;
-  const int avg = sv->n > 0 ? std::max(1, sv->m / sv->n) : 1;
-  (void)avg;
   p.cycles = sv->opts.kernel_cycles > 0 ? sv->opts.kernel_cycles : 2;
   p.interval = sv->opts.relabel_interval > 0 ? sv->opts.relabel_interval : 6;
   p.max_iters = sv->opts.max_iters > 0 ? sv->opts.max_iters : 100000;
@@ -581,13 +579,17 @@ int check_updates_args(dmf_solver *sv, int32_t k, const void *a, const void *b, 
 
 // Host batch -> pinned staging -> device.  Up to kDirectUpdates updates are not
 // copied to the device at all: the lookup reads them once, coalesced, from the
-// pinned buffer, which several threads fill when the batch is not small (1,000
-// updates at R-MAT 20: 53 us a call against 68 with three copies; 32,000: 70
-// against 95; 256,000: 231 against 385).  Larger batches are pipelined: the three arrays are cut into pieces of an eighth of the batch,
-// within [kPieceMin, kPieceMax]; copier threads fill the pinned buffer piece by
-// piece (piece i by thread i mod kStageCopiers, so early pieces finish first)
-// while one issuer thread starts the H2D of each piece as soon as it is in, so
-// the copy engine works while later pieces are still being copied.
+// pinned buffer, which several threads fill when the batch is not small.  A call
+// at R-MAT 20, read in place against copied: 1,000 updates 41 us against 56,
+// 31,000 62 against 83, 126,000 107 against 174, 251,000 180 against 284, 503,000
+// 351 against 433, 1,005,000 1,031 against 682 (the lookup then waits for PCIe
+// longer than the pipelined copy takes).  The limit is well inside: reading in
+// place would still be the faster way for twice as many.
+// Larger batches are pipelined: the three arrays are cut into pieces of an eighth
+// of the batch, within [kPieceMin, kPieceMax]; copier threads fill the pinned
+// buffer piece by piece (piece i by thread i mod kStageCopiers, so early pieces
+// finish first) while one issuer thread starts the H2D of each piece as soon as it
+// is in, so the copy engine works while later pieces are still being copied.
 constexpr size_t kDirectUpdates = 1 << 18;
 constexpr size_t kCopyAlone = 1 << 14;  // batches up to this size are copied by the calling thread
 constexpr size_t kPieceMin = 1 << 15, kPieceMax = 1 << 18;  // updates (128 KiB, 1 MiB of int32)
@@ -753,18 +755,18 @@ int device_updates(dmf_solver *sv, int mode, int32_t k, const int32_t *src, cons
 // pre-sized memory pool or arena, a host that forbids cudaMalloc after start-up,
 // or a deployment that must never grow its footprint mid-flight.  For them
 // dmf_static_maxflow_noalloc keeps all solver scratch (control block, labels,
-// excess, stamps, dead/side marks, vertex queues) in the file-scope array below
+// excess, dead/side marks, vertex queues) in the file-scope array below
 // instead of memory the library allocates; the caller supplies the graph and
 // the residual output in its own device memory.  The array is sized for
-// kNoAllocMaxVertices vertices (about 10 MiB); every GPU that loads the library
+// kNoAllocMaxVertices vertices (about 9 MiB); every GPU that loads the library
 // holds it until the process exits.
 constexpr int kNoAllocMaxVertices = 1 << 18;
 constexpr size_t kNoAllocAlign = 256;
 constexpr size_t na_round(size_t b) { return (b + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
 constexpr size_t kNoAllocV = (size_t)kNoAllocMaxVertices + 1;
 constexpr size_t kNoAllocBytes = na_round(sizeof(Ctrl)) + na_round(4 * kNoAllocV) /* height */ +
-                                 na_round(4 * kNoAllocV) /* stamp */ + na_round(8 * kNoAllocV) /* excess */ +
-                                 na_round(kNoAllocV) /* dead */ + na_round(kNoAllocV) /* side */ +
+                                 na_round(8 * kNoAllocV) /* excess */ + na_round(kNoAllocV) /* dead */ +
+                                 na_round(kNoAllocV) /* side */ +
                                  5 * na_round(4 * kNoAllocV) /* queues */ + 4 * kNoAllocAlign /* unused hub slots */;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -818,7 +820,6 @@ int dmf_static_maxflow_noalloc(int32_t n, int32_t m, const int32_t *d_index, con
     Ctrl *ctrl = (Ctrl *)carve(sizeof(Ctrl));
     Params p{};
     p.height = (int *)carve(4 * N);
-    p.stamp = (int *)carve(4 * N);
     p.excess = (long long *)carve(8 * N);
     p.dead = carve(N);
     p.side = carve(N);
@@ -827,7 +828,8 @@ int dmf_static_maxflow_noalloc(int32_t n, int32_t m, const int32_t *d_index, con
     p.wq[0] = (int *)carve(4 * N);
     p.wq[1] = (int *)carve(4 * N);
     p.aq = (int *)carve(4 * N);
-    p.dq = nullptr;  // static solves never keep a dead set
+    p.stamp = nullptr;  // marks of the local repair and of push-pull, which no static solve has
+    p.dq = nullptr;     // static solves never keep a dead set
     p.dlab = nullptr;
     p.pcur = nullptr;
     p.lq = p.lst = nullptr;
@@ -887,10 +889,9 @@ int dmf_static_maxflow_noalloc(int32_t n, int32_t m, const int32_t *d_index, con
     p.trace_cap = 0;
     p.probe = 0;
     cudaStream_t S = (cudaStream_t)stream;
-    // the array keeps the previous call's contents: the control block and the
-    // worklist stamps must start at zero (everything else is written before use)
+    // the array keeps the previous call's contents: the control block must start
+    // at zero (everything else is written before use)
     CK(cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), S), "memset control");
-    CK(cudaMemsetAsync(p.stamp, 0, 4 * N, S), "memset stamps");
     void *args[] = {&p};
     CK(cudaLaunchCooperativeKernel((const void *)fn, dim3(per_sm * sms), dim3(kBlock), args, 0, S),
        "cooperative launch");

@@ -80,7 +80,11 @@ typedef struct {
   int32_t kernel_cycles;    /* push/relabel cycles per vertex visit; 0 = avg degree
                                (the reference runs avg_deg-1, avg_deg, avg_deg+1,
                                code/dyn_data_bench.cu:529-562) */
-  int32_t relabel_interval; /* push rounds between global relabels; 0 = adaptive */
+  int32_t relabel_interval; /* push rounds between global relabels; 0 = adaptive.  Above
+                               16, as with DMF_FLAG_FIXED_INTERVAL, graphs of high
+                               diameter keep push rounds instead of the barrier-free
+                               push phase, which has none (a 256 x 256 grid: about
+                               nine times as long) */
   int32_t tile;             /* lanes per vertex (1,2,4,8,16,32); 0 = chosen from degree */
   int32_t max_iters;        /* bound on global-relabel iterations per solve; 0 = default */
   int32_t device;           /* CUDA device ordinal; -1 = current device */
@@ -104,8 +108,14 @@ typedef struct {
   int64_t vertices_visited; /* vertex visits (BFS + push) in the last solve */
   int64_t dead_vertices;    /* vertices proven unable to reach t or a deficit */
   double last_ms;           /* device time of the last solve call (CUDA events), from
-                               the batch on the device to the result (host-array
-                               calls: the H2D of the batch is not included) */
+                               the launch to the result.  Host-array calls: the H2D
+                               copy of the batch is not included, but
+                               dmf_apply_updates, dmf_recompute and
+                               dmf_multi_apply_updates do not copy batches of up to
+                               2^18 updates: the kernel reads them from pinned host
+                               memory, and that is included (about 30 us per 10^5
+                               updates).  The _action and _scheduled calls always
+                               copy */
   int32_t grid_blocks;      /* persistent-kernel grid */
   int32_t block_threads;
   int32_t tile;
@@ -235,10 +245,10 @@ int dmf_stats_get(const dmf_solver *sv, dmf_stats *st);
  * saturation, 7 BFS seeds, 8 BFS top-down level, 9 BFS bottom-up level,
  * 10 BFS finalize, 11 push round, 12 flow readout, 13/14 hub push rounds,
  * 15-18 push-pull phase 1, 19 reopen, 20 dead-set pull seeding, 21 pull round,
- * 23 dead-set check, 24 partial revival, 25 capacity claim (duplicate-arc
- * check), 26 barrier-free relabel (deep graphs), 27 barrier-free push phase
- * (counted as one of dmf_stats.push_rounds).  No counterpart in the reference (which
- * times whole calls with cudaEvents, code/dyn_data_bench.cu:246-258). */
+ * 23 dead-set check, 24 partial revival, 26 barrier-free relabel (deep graphs),
+ * 27 barrier-free push phase (counted as one of dmf_stats.push_rounds).  22 and 25
+ * are not used.  No counterpart in the reference (which times whole calls with
+ * cudaEvents, code/dyn_data_bench.cu:246-258). */
 int dmf_trace_get(dmf_solver *sv, int32_t cap, int32_t *kinds, double *t_us,
                   int32_t *count);
 /* Work of each timeline entry: items[i] = vertices in the frontier or worklist
@@ -407,7 +417,7 @@ int dmf_solver_copy_state(dmf_solver *dst, const dmf_solver *src);
  * dmf_graph_from_csr, already validated) and d_res[m] for the residuals of the
  * maximum flow, all in its own device memory; *flow receives the value.  All
  * other scratch lives in one static device array inside the library, sized for
- * n <= 262144 vertices (about 10 MiB, held by every GPU that loads the library
+ * n <= 262144 vertices (about 9 MiB, held by every GPU that loads the library
  * until the process exits); larger n is rejected with DMF_ERR_INVALID_ARG.
  * Every call looks up the array's device address on the current device (the
  * lookup allocates nothing, and stays right if the context was reset).  Calls
