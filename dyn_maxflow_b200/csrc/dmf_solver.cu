@@ -1048,12 +1048,13 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
     if (e == cudaSuccess) e = cudaEventCreate(ev);
   if (e == cudaSuccess) e = cudaStreamSynchronize(S);
   if (e != cudaSuccess) return cuda_fail(e, "solver upload");
-  // Staging for small batches; a larger one grows it in its call.  More up front
-  // is paid for by every solver that never gets such a batch, and is not in
-  // solver_footprint: 2^18 updates on the device and 2^14 pinned took 21 -> 56 ms
-  // of a creation at R-MAT 18 and 6 MiB, and left the first batch of 2 x 10^5
-  // updates, whose pinned buffer had to grow all the same, as long as it was.
-  if ((st = ensure_ubuf(sv, 1024))) return st;
+  // Staging up front: on the device for an eighth of the arcs, up to 2^18 updates,
+  // and for 3% beyond that (a call that has to grow it waits for the device and
+  // for the allocation, up to tens of ms); pinned, which costs ms per MiB to
+  // allocate and only host batches use, for up to 2^14 updates.
+  const size_t some = std::min<size_t>(M / 8, 1 << 18);
+  if ((st = ensure_ubuf(sv, (int)std::max<size_t>({1024, some, M / 32})))) return st;
+  if ((st = ensure_host_ubuf(sv, (int)std::max<size_t>(1024, std::min<size_t>(M / 64, 1 << 14))))) return st;
   // sources (and, for batched instances, roles, instance ids, per-instance flows)
   {
     const std::vector<int> one(1, s);

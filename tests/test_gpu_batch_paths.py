@@ -141,23 +141,3 @@ def test_staging_sizes(dmf, k):
         d = [torch.from_numpy(x).cuda() for x in (src, dst, to)]
         assert sv.apply_updates(src, dst, to) == other.recompute_device(*(x.data_ptr() for x in d), k)
         assert np.array_equal(sv.state()[0], other.state()[0])
-
-
-def test_staging_grows_with_the_batches(dmf):
-    """A new solver holds no staging for batches it may never get (the server's admission does not count any)."""
-    torch = pytest.importorskip("torch")
-    g, s, t = rmat(dmf, 16)
-    k = 200000
-    (big,) = dmf.gen_batches(g, 1, frac=k / (8 << 16), seed=1)
-
-    def free():
-        torch.cuda.synchronize()
-        return torch.cuda.mem_get_info()[0]
-
-    with dmf.Solver(g, s, t) as sv:
-        sv.static_maxflow()
-        made = free()
-        sv.apply_updates(*(x[:1000] for x in big))
-        assert free() == made
-        sv.apply_updates(*big)
-        assert made - free() >= 2 << 20  # five words an update: 4 MB, in allocations of 2 MiB
