@@ -269,6 +269,11 @@ void free_all(dmf_solver *sv) {
 
 constexpr int kTinyVertices = kBlock, kTinyArcs = 8 * kBlock;
 
+// Most updates a new solver has device staging for: what the server reserves for
+// a lane as well.  Staging is not in solver_footprint, so it may not grow with
+// the graph without end (3% of R-MAT 24's arcs would be 330 MB).
+constexpr size_t kStageUpFront = 1 << 20;
+
 int choose_tile(const dmf_opts &o, int n, int m) {
   if (o.tile == 1 || o.tile == 2 || o.tile == 4) return 4;
   if (o.tile == 8 || o.tile == 16 || o.tile == 32) return o.tile;
@@ -1048,12 +1053,13 @@ int setup_solver(dmf_solver *sv, const dmf_graph *g, int32_t s, int32_t t, const
     if (e == cudaSuccess) e = cudaEventCreate(ev);
   if (e == cudaSuccess) e = cudaStreamSynchronize(S);
   if (e != cudaSuccess) return cuda_fail(e, "solver upload");
-  // Staging up front: on the device for an eighth of the arcs, up to 2^18 updates,
-  // and for 3% beyond that (a call that has to grow it waits for the device and
-  // for the allocation, up to tens of ms); pinned, which costs ms per MiB to
-  // allocate and only host batches use, for up to 2^14 updates.
-  const size_t some = std::min<size_t>(M / 8, 1 << 18);
-  if ((st = ensure_ubuf(sv, (int)std::max<size_t>({1024, some, M / 32})))) return st;
+  // Staging up front, 20 bytes an update on the device: for an eighth of the arcs
+  // up to 2^18 updates, for 3% of them beyond that up to kStageUpFront, 20 MiB (a
+  // 1% batch that has to grow it takes 0.57 ms instead of 0.14 at R-MAT 20, now and
+  // then 15 to 30 ms; creating the solver takes no longer with it, 49 ms).  Pinned,
+  // which only host batches use, for up to 2^14 updates.
+  const size_t some = std::max(std::min<size_t>(M / 8, 1 << 18), std::min<size_t>(M / 32, kStageUpFront));
+  if ((st = ensure_ubuf(sv, (int)std::max<size_t>(1024, some)))) return st;
   if ((st = ensure_host_ubuf(sv, (int)std::max<size_t>(1024, std::min<size_t>(M / 64, 1 << 14))))) return st;
   // sources (and, for batched instances, roles, instance ids, per-instance flows)
   {

@@ -141,3 +141,26 @@ def test_staging_sizes(dmf, k):
         d = [torch.from_numpy(x).cuda() for x in (src, dst, to)]
         assert sv.apply_updates(src, dst, to) == other.recompute_device(*(x.data_ptr() for x in d), k)
         assert np.array_equal(sv.state()[0], other.state()[0])
+
+
+def test_staging_of_a_new_solver_is_bounded(dmf):
+    """Staging is not in the footprint that the server admits by: 2^20 updates of five words, whatever the graph."""
+    torch = pytest.importorskip("torch")
+    g, s, t = dmf.gen_rmat(21, 18 << 21, seed=21, cap_lo=1, cap_hi=1000)
+    index, adj, w, _ = g.arrays()
+    assert len(adj) // 32 > (1 << 20) + (1 << 19)
+    pick = np.random.default_rng(21).permutation(len(adj))[:(1 << 20) + (1 << 19)]
+    src, dst = arcs_of(g, pick)
+    x = [torch.from_numpy(a).cuda() for a in (src, dst, w[pick])]  # sets what is there already
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    with dmf.Solver(g, s, t) as sv:
+        flow = sv.static_maxflow()
+        made = free()
+        assert sv.apply_updates_device(*(a.data_ptr() for a in x), 1 << 20) == flow
+        assert free() == made
+        assert sv.apply_updates_device(*(a.data_ptr() for a in x), len(pick)) == flow
+        assert 8 << 20 <= made - free() <= 16 << 20  # 30 MiB in the place of 20
