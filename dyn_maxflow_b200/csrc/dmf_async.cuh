@@ -29,9 +29,10 @@ constexpr int kAsyncWin = 4;
 constexpr int kQuietPolls = 8;
 // A sink's row longer than this is relaxed by a level-synchronous level at the
 // start of every relabel, over the whole grid, before the barrier-free phase: one
-// warp takes it 128 arcs in about 0.8 us, the seeds with their frontier and the
-// level about 25 us for any length.  Segmentation graphs (every vertex of a grid
-// joined to s and t), static solve with the level / without / barriers throughout:
+// warp takes about 1 ms for 65,536 arcs (from the totals below; the push phase gets
+// as long again), the seeds with their frontier and the level tens of us for any
+// length.  Segmentation graphs (every vertex of a grid joined to s and t), static
+// solve with the level / without / barriers throughout:
 // 1,024 arcs 0.96 / 0.98 / 1.9 ms, 2,304 arcs 0.65 / 0.75 / 1.5, 65,536 arcs 1.05 /
 // 6.6 / 3.4, 262,144 arcs 3.0 / 16 / 7.2.  Other long rows stay with one warp: a
 // hub of 100,000 arcs on a ladder, 43 ms against 220 with barriers throughout.
@@ -147,8 +148,9 @@ __device__ __forceinline__ bool async_quiet(AsyncShared &sh, AsyncIdle &st, bool
 
 // Relaxes the tails of a long row's residual in-arcs, by a whole warp, kRelaxBatch
 // arcs a lane with their loads in flight together.  No other warp helps with the
-// row, so everything behind it waits (65,536 arcs: about 0.5 ms; one arc a lane at
-// a time about 2 ms; 8 were no faster than 4).
+// row, so everything behind it waits: static solve of a 256 x 256 segmentation
+// graph, its sink's row of 65,536 arcs taken this way, 8.4 ms with one arc a lane,
+// 6.3 with 4, 6.3 with 8.
 constexpr int kRelaxBatch = 4;
 
 __device__ __forceinline__ void async_relax_row(const Params &p, int v, int h, LStats &ls) {
